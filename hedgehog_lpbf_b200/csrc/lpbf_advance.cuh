@@ -31,12 +31,12 @@
 // just off the field holds its neighbour's cells in reverse order); rows of
 // the chunk's own halo are computed there too and only masked out of the
 // store and the reduction (a value outside a level's valid range only ever
-// feeds rows that are themselves outside the next level's range).  Every
-// other box runs the general body, which handles the top and bottom edges,
-// fixed-value boundaries, partial ownership and the Gaussian source
-// (evaluated out of line, so exp is not replicated).  Both bodies evaluate
-// every cell with the same function, so results depend neither on the body
-// nor on K, H or the task order.
+// feeds rows that are themselves outside the next level's range).  Interior
+// boxes that meet the source run the same body with the source product added.
+// Every other box runs the general body, which handles the top and bottom
+// edges, fixed-value boundaries, partial ownership and the source beside
+// them.  All bodies evaluate every cell with the same functions, so results
+// depend neither on the body nor on K, H or the task order.
 //
 // Reduction.  For every level (= time step) each lane keeps the peak T with
 // its flat index, and each warp the molten row extent (warp vote), over owned
@@ -163,18 +163,44 @@ __device__ __forceinline__ double cell_core_src(double T, double L, double R, do
     return __dadd_rn(T, __dadd_rn(cell_net<SQ>(T, L, R, U, D, h), S));
 }
 
-// Gaussian source increment of a lane's four cells starting at column x0
-// (out of line: the exp code exists once in the binary).
-static __device__ __noinline__ double4 source4(int x0, double dy2, double x_l, double cs, double dx,
-                                        double m2r, double r2_cut) {
-    double S[4];
+// The Gaussian source increment of a cell is the product of a row factor
+// cs exp(-2 yd^2 / r0^2) and a column factor exp(-2 xd^2 / r0^2), each zero
+// beyond the truncation radius: two short tables replace an exp per cell and
+// step.  A task fills its column factors once (src_columns) and each box its
+// row factors, one (row, level) per lane; a cell then costs one
+// multiply.  Every kernel forms the increment from these two functions and
+// src_product, so all paths stay bit-identical.  Against long double over
+// spots of 24-70 um on grids of 120-8192 columns the product's error equals
+// the single exp's (largest 1.152e-13 of the peak against 1.153e-13: both
+// come from rounding the positions).  Out of line: the exp code exists once
+// in the binary.  What it bounds: a task on the source is a serial chain that
+// ends the launch of a small or middling field.  With an exp per cell in the
+// general body a launch of 3 steps at 2048^2 took 69 us (the SMs idle for
+// 54 % of it, waiting for those tasks), with the product and the plain body
+// 49 us; 256 mixed fields 1.62 -> 1.43 ms per launch; 8192^2 unchanged.
+static __device__ __noinline__ double src_factor(double d, double m2r, double r2_cut) {
+    const double d2 = __dmul_rn(d, d);
+    return d2 < r2_cut ? exp(__dmul_rn(m2r, d2)) : 0.0;
+}
+// Column factors of the four cells from column x0.
+static __device__ __noinline__ double4 src_columns(int x0, double x_l, double dx, double m2r,
+                                                   double r2_cut) {
+    double f[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-        const double xd = __dsub_rn(__dmul_rn((double)(x0 + v), dx), x_l);
-        const double r2 = __dadd_rn(__dmul_rn(xd, xd), dy2);
-        S[v] = (r2 < r2_cut) ? cs * exp(__dmul_rn(m2r, r2)) : 0.0;
+        const double d = __dsub_rn(__dmul_rn((double)(x0 + v), dx), x_l);
+        const double d2 = __dmul_rn(d, d);
+        f[v] = d2 < r2_cut ? exp(__dmul_rn(m2r, d2)) : 0.0;
     }
-    return make_double4(S[0], S[1], S[2], S[3]);
+    return make_double4(f[0], f[1], f[2], f[3]);
+}
+// Row factor with the amplitude cs folded in; zero (not NaN) off the source.
+__device__ __forceinline__ double src_row(int row, const LaserSub& l, const Coef& c) {
+    const double f = src_factor(__dsub_rn(__dmul_rn((double)row, c.dy), l.y_l), c.m2r, c.r2_cut);
+    return f > 0.0 ? __dmul_rn(l.cs, f) : 0.0;
+}
+__device__ __forceinline__ double src_product(double row_f, double col_f) {
+    return col_f > 0.0 ? __dmul_rn(row_f, col_f) : 0.0;
 }
 
 // 32-byte stores of level-K values.  They carry no "memory" clobber: the
@@ -238,6 +264,13 @@ struct WarpStrip {
     int msrc;                            // lane whose cells this lane mirrors (own lane if none)
     bool fast_ok;                        // the task may use the fast body at all
     bool incl;                           // this task also examines values equal to the lane peak
+
+    // Source factors of a task that meets the source: the column factors of
+    // the lane's cells, four per level, filled once per task; then one row
+    // factor per lane and box (lane 3 (t - 1) + P: level t's row j + P - t;
+    // zero off the source).  In local memory (L1): registers for them would
+    // be taken from every other task.
+    double* srcf;
 
     double w0[3][V];                     // level-0 window (slot = row % 3)
     double w[K > 1 ? K - 1 : 1][3][V];   // windows of levels 1..K-1
@@ -309,6 +342,8 @@ struct WarpStrip {
     }
 
     __device__ __forceinline__ void run_task(int task) {
+        double factors[K * V + 1];
+        srcf = factors;
         const int nx = p.c.nx, ny = p.c.ny;
         const int strip = task % p.nstrips, chunk = task / p.nstrips;
         // A warp draws tasks in increasing order, so its earlier tasks lie in
@@ -351,6 +386,7 @@ struct WarpStrip {
             }
         }
         const int jlast = y1 - 1 + K;
+        if (src_strip && y0 - K <= p.band_hi && y1 + K >= p.band_lo) fill_columns();
         // per-box thresholds change only when an exact pass moves a peak
         if constexpr (REDUCE) set_thresholds();
         for (int b = 0, j = jy0; j <= jlast && !failed; ++b, j += ADV_R) {
@@ -360,16 +396,26 @@ struct WarpStrip {
                 if (failed) break;
             }
             // computed rows of this box: j-K .. j+1 over all levels
-            const bool fast = fast_ok && j - K >= 1 && j + 1 <= ny - 2 &&
-                              (!src_strip || j + 1 < p.band_lo || j - K > p.band_hi);
+            const bool src_box = src_strip && j + 1 >= p.band_lo && j - K <= p.band_hi;
+            const bool interior = fast_ok && j - K >= 1 && j + 1 <= ny - 2;
+            const bool fast = interior && !src_box;
             if (fast && j < jend) {
                 if constexpr (SQM == 2) {
-                    if (h.sq) fast_box<true>(j, st);
-                    else      fast_box<false>(j, st);
+                    if (h.sq) fast_box<true, false>(j, st);
+                    else      fast_box<false, false>(j, st);
                 } else {
-                    fast_box<SQM == 1>(j, st);
+                    fast_box<SQM == 1, false>(j, st);
+                }
+            } else if (interior && !mir && j < jend) {
+                fill_rows(j, src_box);
+                if constexpr (SQM == 2) {
+                    if (h.sq) fast_box<true, true>(j, st);
+                    else      fast_box<false, true>(j, st);
+                } else {
+                    fast_box<SQM == 1, true>(j, st);
                 }
             } else {
+                fill_rows(j, src_box);
                 general_row<0>(j, st, jlast);
                 general_row<1>(j + 1, st, jlast);
                 general_row<2>(j + 2, st, jlast);
@@ -464,21 +510,25 @@ struct WarpStrip {
         }
     }
 
-    template <bool SQ>
+    // SRC: the box meets the source; its cells get the source product added
+    // (zero factors where the beam is off).
+    template <bool SQ, bool SRC>
     __device__ __forceinline__ void fast_box(int j, const double* st) {
-        fast_row<0, SQ>(j, st);
-        fast_row<1, SQ>(j + 1, st);
-        fast_row<2, SQ>(j + 2, st);
+        fast_row<0, SQ, SRC>(j, st);
+        fast_row<1, SQ, SRC>(j + 1, st);
+        fast_row<2, SQ, SRC>(j + 2, st);
     }
 
-    template <int P, bool SQ>
+    template <int P, bool SQ, bool SRC>
     __device__ __forceinline__ void fast_row(int jj, const double* st) {
         load_row0<P>(jj, st, win<0>()[P]);
-        if (mir) mirror_fix(win<0>()[P]);
-        fast_level<P, 1, SQ>(jj);
+        if constexpr (!SRC) {
+            if (mir) mirror_fix(win<0>()[P]);
+        }
+        fast_level<P, 1, SQ, SRC>(jj);
     }
 
-    template <int P, int T, bool SQ>
+    template <int P, int T, bool SQ, bool SRC>
     __device__ __forceinline__ void fast_level(int jj) {
         if constexpr (T <= K) {
             constexpr int su = mod3(P - T - 1), sc = mod3(P - T), sd = mod3(P - T + 1);
@@ -489,10 +539,26 @@ struct WarpStrip {
             double Lo, Ro;
             neighbours(ce, Lo, Ro);
             double nv[V];
-            nv[0] = cell_core<SQ>(ce[0], Lo, ce[1], up[0], dn[0], h);
-            nv[1] = cell_core<SQ>(ce[1], ce[0], ce[2], up[1], dn[1], h);
-            nv[2] = cell_core<SQ>(ce[2], ce[1], ce[3], up[2], dn[2], h);
-            nv[3] = cell_core<SQ>(ce[3], ce[2], Ro, up[3], dn[3], h);
+            if constexpr (SRC) {
+                // A warp sync per level keeps the compiler from interleaving the
+                // levels (as it should in the plain box): the source's
+                // temporaries on top would spill (84 bytes at depth 3).
+                __syncwarp();
+                const volatile double* sf = srcf;
+                const double rf = __shfl_sync(0xffffffffu, sf[K * V], 3 * (T - 1) + P);
+                double S[V];
+#pragma unroll
+                for (int v = 0; v < V; ++v) S[v] = src_product(rf, sf[(T - 1) * V + v]);
+                nv[0] = cell_core_src<SQ>(ce[0], Lo, ce[1], up[0], dn[0], S[0], h);
+                nv[1] = cell_core_src<SQ>(ce[1], ce[0], ce[2], up[1], dn[1], S[1], h);
+                nv[2] = cell_core_src<SQ>(ce[2], ce[1], ce[3], up[2], dn[2], S[2], h);
+                nv[3] = cell_core_src<SQ>(ce[3], ce[2], Ro, up[3], dn[3], S[3], h);
+            } else {
+                nv[0] = cell_core<SQ>(ce[0], Lo, ce[1], up[0], dn[0], h);
+                nv[1] = cell_core<SQ>(ce[1], ce[0], ce[2], up[1], dn[1], h);
+                nv[2] = cell_core<SQ>(ce[2], ce[1], ce[3], up[2], dn[2], h);
+                nv[3] = cell_core<SQ>(ce[3], ce[2], Ro, up[3], dn[3], h);
+            }
             const int r = jj - T;
             // Rows outside [y0, y1) are this chunk's halo: computed (their
             // values only ever feed other halo rows) but not stored or reduced.
@@ -510,8 +576,26 @@ struct WarpStrip {
             // task (values of no use here, which would only trigger empty
             // exact passes).
             if constexpr (REDUCE) row_stats_fast<T - 1, P>(nv, owned_row);
-            fast_level<P, T + 1, SQ>(jj);
+            fast_level<P, T + 1, SQ, SRC>(jj);
         }
+    }
+
+    // ---- source factors ----------------------------------------------------
+    __device__ __noinline__ static void columns_to(double* out, int xl, const AdvParams& p) {
+#pragma unroll 1
+        for (int t = 0; t < K; ++t) {
+            const double4 f = src_columns(xl, p.las[t].x_l, p.c.dx, p.c.m2r, p.c.r2_cut);
+            out[t * V] = f.x; out[t * V + 1] = f.y; out[t * V + 2] = f.z; out[t * V + 3] = f.w;
+        }
+    }
+    __device__ __forceinline__ void fill_columns() { columns_to(srcf, xl, p); }
+    __device__ __forceinline__ void fill_rows(int j, bool src_box) {
+        double f = 0.0;
+        if (src_box) {
+            const int t = min(lane / 3, K - 1), P = lane % 3;
+            f = src_row(j + P - (t + 1) + p.row0, p.las[t], p.c);
+        }
+        srcf[K * V] = f;
     }
 
     // ---- general body ----------------------------------------------------
@@ -547,7 +631,7 @@ struct WarpStrip {
                     for (int v = 0; v < V; ++v) wn[sd][v] = wn[sc][v];
                 }
                 double nv[V];
-                compute_row_general(wn[su], wn[sc], wn[sd], r, p.las[T - 1], nv);
+                compute_row_general<P, T>(wn[su], wn[sc], wn[sd], r, nv);
                 // keep the mirror lanes exact for later fast boxes (the source
                 // term and the edge patch are not mirror-symmetric off the field)
                 if constexpr (T < K) {
@@ -586,9 +670,9 @@ struct WarpStrip {
         return xl >= x0 && xl < x0 + ADV_WOUT && xl < p.c.nx;
     }
 
+    template <int P, int T>
     __device__ __forceinline__ void compute_row_general(const double* up, const double* ce,
-                                                        const double* dn, int r,
-                                                        const LaserSub& las, double* nv) {
+                                                        const double* dn, int r, double* nv) {
         const Coef& c = p.c;
         const int nx = c.nx, ny = c.ny;
         if (c.bc == 1 && (r == 0 || r == ny - 1)) {
@@ -607,12 +691,13 @@ struct WarpStrip {
                 if (xl + v == nx - 1) R[v] = ce[v];
             }
         }
-        const double yd = __dsub_rn(__dmul_rn((double)(r + p.row0), c.dy), las.y_l);
-        const double dy2 = __dmul_rn(yd, yd);
-        const bool src = las.cs != 0.0 && dy2 < c.r2_cut && src_strip;
-        double4 S4 = make_double4(0.0, 0.0, 0.0, 0.0);
-        if (src) S4 = source4(xl, dy2, las.x_l, las.cs, c.dx, c.m2r, c.r2_cut);
-        const double S[V] = {S4.x, S4.y, S4.z, S4.w};
+        const double rf = __shfl_sync(0xffffffffu, srcf[K * V], 3 * (T - 1) + P);
+        const bool src = rf != 0.0;
+        double S[V] = {0.0, 0.0, 0.0, 0.0};
+        if (src) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) S[v] = src_product(rf, srcf[(T - 1) * V + v]);
+        }
         if (c.same_T) {
 #pragma unroll
             for (int v = 0; v < V; ++v)
@@ -726,37 +811,54 @@ struct WarpStrip {
     __device__ __forceinline__ void exact_rows(const double (&x)[3][V], int j, unsigned rows) {
         const int nx = p.c.nx;
         const bool ol = owned_lane();
-        double m = -INFINITY;
-        long long a = -1;
-        bool nonfinite = false;
+        // bit P: row P holds a molten cell; bit 3: a NaN or infinite cell
+        unsigned flags = 0u;
+        double rm[3];
+        int ra[3];
 #pragma unroll
         for (int P = 0; P < 3; ++P) {
             const int r = j + P - T;
             const bool cand = ((rows >> P) & 1u) && r >= y0 && r < y1 && ol;
-            bool hot = false;
+            double c[V];
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 const bool ok = cand && xl + v < nx;
                 const double val = x[P][v];
-                // rows, then columns, ascend: the first maximum has the
-                // smallest flat index (NaN never wins)
-                const bool take = ok && val > m;
-                m = take ? val : m;
-                a = take ? (long long)(r + p.row0) * nx + xl + v : a;
-                hot |= ok && val > p.c.Tm;
-                nonfinite |= ok && !(fabs(val) < INFINITY);
+                flags |= ok && val > p.c.Tm ? 1u << P : 0u;
+                flags |= ok && !(fabs(val) < INFINITY) ? 8u : 0u;
+                // NaN never wins
+                c[v] = ok && val > -INFINITY ? val : -INFINITY;
             }
-            if (__any_sync(0xffffffffu, hot) && lane == 0) {
-                rs->ymn[T - 1] = min(rs->ymn[T - 1], r + p.row0);
-                rs->ymx[T - 1] = max(rs->ymx[T - 1], r + p.row0);
-            }
+            // first maximum of the row: pairs, then the pairs' winners (a
+            // strict '>' keeps the smaller index), so the compares chain
+            // four deep over the box instead of twelve
+            const bool h01 = c[1] > c[0], h23 = c[3] > c[2];
+            const double m01 = h01 ? c[1] : c[0], m23 = h23 ? c[3] : c[2];
+            const bool hh = m23 > m01;
+            rm[P] = hh ? m23 : m01;
+            ra[P] = P * V + (hh ? (h23 ? 3 : 2) : (h01 ? 1 : 0));
         }
-        // a NaN or infinite temperature is reported, never trapped on; the
-        // peak keeps the reference rule (NaN never wins)
-        if (__any_sync(0xffffffffu, nonfinite) && lane == 0 && p.err) atomicOr(p.err, 2u);
+        const bool t1 = rm[1] > rm[0];
+        double m = t1 ? rm[1] : rm[0];
+        int a3 = t1 ? ra[1] : ra[0];
+        const bool t2 = rm[2] > m;
+        m = t2 ? rm[2] : m;
+        a3 = t2 ? ra[2] : a3;
+        const long long a = (long long)(j + a3 / V - T + p.row0) * nx + xl + a3 % V;
+        flags = __reduce_or_sync(0xffffffffu, flags);
+        if (flags != 0u && lane == 0) {
+            const int r0 = j - T + p.row0;
+            if (flags & 7u) {
+                rs->ymn[T - 1] = min(rs->ymn[T - 1], r0 + __ffs(flags & 7u) - 1);
+                rs->ymx[T - 1] = max(rs->ymx[T - 1], r0 + 31 - __clz(flags & 7u));
+            }
+            // a NaN or infinite temperature is reported, never trapped on;
+            // the peak keeps the reference rule (NaN never wins)
+            if ((flags & 8u) && p.err) atomicOr(p.err, 2u);
+        }
         const double pk = rs->tmx[T - 1][lane];
         // an equal peak (inclusive task) moves only to a smaller index
-        if (m > pk || (incl && m == pk && a < rs->arg[T - 1][lane])) {
+        if (m > pk || (incl && m == pk && m > -INFINITY && a < rs->arg[T - 1][lane])) {
             rs->tmx[T - 1][lane] = m;
             rs->arg[T - 1][lane] = a;
         }

@@ -162,6 +162,8 @@ struct FkStrip {
 
     int x0, xs, xl, y0, y1, jy0, jend, nbox, issued;
     bool edge, failed, src_strip;
+    double rowf;                       // this box's row factors of the source (as WarpStrip)
+    double* colf;                      // the task's column factors, four per level
 
     float wh0[3][V], wl0[3][V];
     float wh[K > 1 ? K - 1 : 1][3][V], wl[K > 1 ? K - 1 : 1][3][V];
@@ -207,7 +209,18 @@ struct FkStrip {
         return xl >= x0 && xl < x0 + ADV_WOUT && xl < p.c.nx;
     }
 
+    __device__ __noinline__ static void columns_to(double* out, int xl, const FkParams& p) {
+#pragma unroll 1
+        for (int t = 0; t < K; ++t) {
+            const double4 f = src_columns(xl, p.las[t].x_l, p.c.dx, p.c.m2r, p.c.r2_cut);
+            out[t * V] = f.x; out[t * V + 1] = f.y; out[t * V + 2] = f.z; out[t * V + 3] = f.w;
+        }
+    }
+
     __device__ __forceinline__ void run_task(int task) {
+        double cols[K * V];
+        colf = cols;
+        rowf = 0.0;
         const int nx = p.c.nx, ny = p.c.ny;
         const int strip = task % p.nstrips, chunk = task / p.nstrips;
         x0 = strip * ADV_WOUT;
@@ -235,6 +248,7 @@ struct FkStrip {
             for (int b = 0; b < pre; ++b) issue(b);
         }
         const int jlast = y1 - 1 + K;
+        if (src_strip && y0 - K <= p.band_hi && y1 + K >= p.band_lo) columns_to(colf, xl, p);
         // per-box thresholds change only when an exact pass moves a peak
         if constexpr (REDUCE) set_thresholds();
         for (int b = 0, j = jy0; j <= jlast && !failed; ++b, j += ADV_R) {
@@ -252,9 +266,14 @@ struct FkStrip {
             }
             // mirror-edge strips too: row_update patches the edge cells'
             // outer neighbours itself (nx a multiple of 4: whole lanes)
+            const bool src_box = src_strip && j + 1 >= p.band_lo && j - K <= p.band_hi;
             const bool fast = (!edge || (p.c.bc == 0 && (p.c.nx & 3) == 0)) &&
-                              j - K >= 1 && j + 1 <= ny - 2 &&
-                              (!src_strip || j + 1 < p.band_lo || j - K > p.band_hi);
+                              j - K >= 1 && j + 1 <= ny - 2 && !src_box;
+            rowf = 0.0;
+            if (src_box) {
+                const int t = min(lane / 3, K - 1);
+                rowf = src_row(j + lane % 3 - (t + 1), p.las[t], p.c);
+            }
             if (fast && j < jend) {
                 fast_row<0>(j, st);
                 fast_row<1>(j + 1, st);
@@ -403,14 +422,12 @@ struct FkStrip {
 #pragma unroll
                     for (int v = 0; v < V; ++v) { oh[v] = p.f.Tedge_hi; ol[v] = p.f.Tedge_lo; }
                 } else {
-                    const LaserSub& las = p.las[T - 1];
-                    const double yd = __dsub_rn(__dmul_rn((double)r, p.c.dy), las.y_l);
-                    const double dy2 = __dmul_rn(yd, yd);
+                    const double rf = __shfl_sync(0xffffffffu, rowf, 3 * (T - 1) + P);
                     float S[V] = {0.f, 0.f, 0.f, 0.f};
-                    if (las.cs != 0.0 && dy2 < p.c.r2_cut && src_strip) {
-                        const double4 s4 = source4(xl, dy2, las.x_l, las.cs, p.c.dx, p.c.m2r,
-                                                   p.c.r2_cut);
-                        S[0] = (float)s4.x; S[1] = (float)s4.y; S[2] = (float)s4.z; S[3] = (float)s4.w;
+                    if (rf != 0.0) {
+#pragma unroll
+                        for (int v = 0; v < V; ++v)
+                            S[v] = (float)src_product(rf, colf[(T - 1) * V + v]);
                     }
                     row_update(ah[su], al[su], ah[sc], al[sc], ah[sd], al[sd], S, oh, ol);
                     if (edge && p.c.bc == 1) {
