@@ -31,14 +31,18 @@ struct NvtxRange {
 
 constexpr int MAX_CTAS = 2048;     // most CTAs a reducing launch may use
 
-// Device workspace.  The counter and error word sit in the first 256 bytes;
-// per-CTA partials follow.
+// Device workspace.  The counters and error word sit in the first 256 bytes;
+// per-CTA partials follow, then the resident kernel's progress flags.
+constexpr int WS_PARTS = 40960;    // partial records (resident kernel: 256 steps x 160 tiles)
+static_assert(WS_PARTS >= MAX_CTAS * KMAX, "records of one launch");
 struct Workspace {
     unsigned int counter;          // last-CTA ticket
     unsigned int err;              // error word
     unsigned int tasks;            // dynamic task counter
-    unsigned int pad[61];
-    Partial parts[MAX_CTAS * KMAX];
+    unsigned int barrier;          // arrivals of the resident kernel's final fold
+    unsigned int pad[60];
+    Partial parts[WS_PARTS];
+    unsigned int flags[160 * 8];   // zero between launches
 };
 static_assert(offsetof(Workspace, parts) == 256, "workspace header");
 
@@ -98,6 +102,18 @@ cudaError_t launch_advance(int K, const double* Tin, double* Tout, const Coef& c
                            Partial* ref_out, long long ref_nparts, int rows,
                            cudaStream_t stream, const RowWindow* win = nullptr,
                            int parts_cap = MAX_CTAS * KMAX);
+
+// Many steps of a field small enough to stay in shared memory in one launch
+// (lpbf_resident.cuh).  resident_plan: false when the field does not fit;
+// `steps` is the most steps of one launch.  launch_resident advances n_steps
+// (<= steps) from Tin into Tout; Tin_rw is Tin, which carries the tiles' rims
+// between exchanges (its contents are lost).
+constexpr int RES_MAX_STEPS = 256; // most steps of one launch
+struct ResPlan { int V, NR, gx, gy, K, hx, hy, steps; };
+bool resident_plan(int nx, int ny, int n_steps, ResPlan* out);
+cudaError_t launch_resident(const ResPlan& pl, const double* Tin, double* Tout, double* Tin_rw,
+                            const Coef& c, const LaserSub* las, int n_steps, Partial* ring,
+                            Workspace* ws, cudaStream_t stream);
 
 // Extended-physics (phys == 1) single step, one thread per cell, with the
 // same reduction outputs as launch_advance.

@@ -12,8 +12,9 @@
  *   lpbf_b200_advance   the per-step loop of GpuStepTask::execute
  *                       (include/gpu_step_task.hpp:149-197): step + reduce +
  *                       finalize for `n_steps` Ticks of a plan, in
- *                       ceil(n_steps / depth) launches instead of 2-4
- *                       launches per step.
+ *                       ceil(n_steps / depth) launches (fields of up to
+ *                       about 1.9 M cells at automatic depth: one per 256
+ *                       steps) instead of 2-4 launches per step.
  * ---------------------------------------------------------------------------
  */
 #ifndef LPBF_B200_H
@@ -88,7 +89,8 @@ int lpbf_b200_advance(double* T_a, double* T_b, const StepConst* k,
                       Partial* ring, void* work, size_t work_bytes,
                       cudaStream_t stream, int* result_in_b);
 
-/* Number of launches lpbf_b200_advance issues for these arguments. */
+/* Number of launches lpbf_b200_advance issues for these arguments (with a
+ * workspace; it depends on the current device). */
 int lpbf_b200_advance_launches(int nx, int ny, int n_steps, const lpbf_b200_opts* opts);
 
 /* A row strip of a larger field: the buffers hold rows row0 .. row0+k->ny-1
@@ -120,7 +122,8 @@ int lpbf_b200_advance_rows(const double* T_in, double* T_out, const StepConst* k
                            size_t work_bytes, cudaStream_t stream);
 
 /* Copy the workspace error word to *err (synchronizes `stream`); bit 0 means
- * a TMA wait exceeded its time limit and the launch stopped early; bit 1
+ * a bounded wait (a TMA copy, or a neighbouring tile of the resident kernel)
+ * ran out and the field is incomplete; bit 1
  * means a computed temperature was NaN or infinite (baseline FP64 advance
  * with a ring; the Partials ignore NaN as the reference does).  The word
  * accumulates until lpbf_b200_workspace_init clears it. */
