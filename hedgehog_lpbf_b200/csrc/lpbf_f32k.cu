@@ -61,6 +61,9 @@ cudaError_t launch_fk(const float* hi_in, const float* lo_in, float* hi_out, flo
     std::memset(&p, 0, sizeof(p));
     p.c = c;
     p.f = f;
+    p.f2 = FkCoef2{p2_host(f.ax), p2_host(f.ay), p2_host(-f.cls), p2_host(-f.crad),
+                   p2_host(-f.Ta4), p2_host(f.clsTa), p2_host(f.Ta_hi), p2_host(f.Ta_lo),
+                   p2_host(-4.0f), p2_host(-2.0f)};
     for (int t = 0; t < K; ++t) p.las[t] = las[t];
     laser_band(c, las, K, &p.band_lo, &p.band_hi, &p.bandx_lo, &p.bandx_hi);
     p.nstrips = (c.nx + ADV_WOUT - 1) / ADV_WOUT;

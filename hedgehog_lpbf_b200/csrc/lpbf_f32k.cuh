@@ -28,6 +28,8 @@
 #pragma once
 #include <stddef.h>
 
+#include <cstring>
+
 #include "lpbf_advance.cuh"
 
 namespace lpbf_b200 {
@@ -51,6 +53,68 @@ __device__ __forceinline__ void st_global_v4f_pred(float* p, const float* v, boo
                  : "memory");
 }
 
+// ---- packed pairs of f32 -----------------------------------------------------
+// sm_100a executes two f32 operations per instruction on a 64-bit register
+// pair, each rounded as its scalar form.  These kernels are bound by
+// instruction issue, so the fast body holds and updates its four cells per
+// lane as two pairs; only what needs a neighbour across a pair's seam stays
+// scalar (the horizontal differences and sums, whose results land in pairs).
+typedef unsigned long long p2;
+__device__ __forceinline__ p2 p2_pack(float a, float b) {
+    p2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float p2_a(p2 v) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return a;
+}
+__device__ __forceinline__ float p2_b(p2 v) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return b;
+}
+__device__ __forceinline__ p2 p2_add(p2 a, p2 b) {
+    p2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ p2 p2_mul(p2 a, p2 b) {
+    p2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ p2 p2_fma(p2 a, p2 b, p2 c) {
+    p2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ p2 p2_sub(p2 a, p2 b) {
+    p2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+inline p2 p2_host(float v) {            // both halves v
+    unsigned int b;
+    std::memcpy(&b, &v, sizeof(b));
+    return ((p2)b << 32) | b;
+}
+
+// FkCoef's constants as pairs, the loss coefficients negated (rounding is
+// symmetric: the fast body adds -loss).
+struct FkCoef2 {
+    p2 ax, ay, ncls, ncrad, nTa4, clsTa, Ta_hi, Ta_lo, m4, m2;
+};
+
+// 16-byte store of two pairs issued under a predicate, as st_global_v4f_pred.
+__device__ __forceinline__ void st_global_v2_pred(float* p, const p2* v, bool pred) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\t"
+                 "@q st.global.v2.b64 [%0], {%1, %2};\n\t}"
+                 :: "l"(p), "l"(v[0]), "l"(v[1]), "r"((int)pred)
+                 : "memory");
+}
+
 struct FkCoef {
     float ax, ay, cls, crad;
     float Ta_hi, Ta_lo, Ta4;       // linear-loss reference T as a pair; Ta4 = f4(Tamb)
@@ -61,6 +125,7 @@ struct FkCoef {
 struct FkParams {
     Coef c;                        // geometry, source and reduction constants
     FkCoef f;
+    FkCoef2 f2;
     LaserSub las[KMAX];
     int band_lo, band_hi, bandx_lo, bandx_hi;
     int nstrips, nchunks, H, ntasks;
@@ -161,12 +226,13 @@ struct FkStrip {
     const int lane;
 
     int x0, xs, xl, y0, y1, jy0, jend, nbox, issued;
-    bool edge, failed, src_strip;
+    bool edge, failed, src_strip, own_all;
+    bool first_col, last_col;          // the lane holds the field's first / last column (mirror)
     double rowf;                       // this box's row factors of the source (as WarpStrip)
     double* colf;                      // the task's column factors, four per level
 
-    float wh0[3][V], wl0[3][V];
-    float wh[K > 1 ? K - 1 : 1][3][V], wl[K > 1 ? K - 1 : 1][3][V];
+    p2 wh0[3][2], wl0[3][2];           // windows: a lane's four cells as two pairs
+    p2 wh[K > 1 ? K - 1 : 1][3][2], wl[K > 1 ? K - 1 : 1][3][2];
     float thr_h[K], thr_l[K];
     bool hit[K];
     double (*s_tmx)[32];
@@ -242,6 +308,9 @@ struct FkStrip {
         nbox = (jend - jy0 + ADV_R - 1) / ADV_R;
         edge = (xs <= 0) || (xs + ADV_COLS > nx - 1);
         src_strip = !(xs + ADV_COLS <= p.bandx_lo || xs > p.bandx_hi);
+        own_all = owned_lane();            // nx is a multiple of 4: whole lanes
+        first_col = p.c.bc == 0 && xl == 0;
+        last_col = p.c.bc == 0 && xl + V == nx;
         issued = 0;
         if (lane == 0) {
             const int pre = min(ADV_S, nbox);
@@ -304,22 +373,26 @@ struct FkStrip {
 
     template <int P>
     __device__ __forceinline__ void load_row0(const float* st) {
-        const float4 h = *reinterpret_cast<const float4*>(st + P * ADV_COLS + 4 * lane);
-        wh0[P][0] = h.x; wh0[P][1] = h.y; wh0[P][2] = h.z; wh0[P][3] = h.w;
+        const ulonglong2 h = *reinterpret_cast<const ulonglong2*>(st + P * ADV_COLS + 4 * lane);
+        wh0[P][0] = h.x; wh0[P][1] = h.y;
         if constexpr (COMP) {
-            const float4 l =
-                *reinterpret_cast<const float4*>(st + (ADV_R + P) * ADV_COLS + 4 * lane);
-            wl0[P][0] = l.x; wl0[P][1] = l.y; wl0[P][2] = l.z; wl0[P][3] = l.w;
+            const ulonglong2 l =
+                *reinterpret_cast<const ulonglong2*>(st + (ADV_R + P) * ADV_COLS + 4 * lane);
+            wl0[P][0] = l.x; wl0[P][1] = l.y;
         }
     }
 
     template <int T>
-    __device__ __forceinline__ float (&winh())[3][V] {
+    __device__ __forceinline__ p2 (&winh())[3][2] {
         if constexpr (T == 0) return wh0; else return wh[T - 1];
     }
     template <int T>
-    __device__ __forceinline__ float (&winl())[3][V] {
+    __device__ __forceinline__ p2 (&winl())[3][2] {
         if constexpr (T == 0) return wl0; else return wl[T - 1];
+    }
+
+    __device__ __forceinline__ static void unpack(const p2* w, float* d) {
+        d[0] = p2_a(w[0]); d[1] = p2_b(w[0]); d[2] = p2_a(w[1]); d[3] = p2_b(w[1]);
     }
 
     // One row of level T from the three rows (up, centre, down) of level T-1
@@ -341,8 +414,7 @@ struct FkStrip {
             }
 #pragma unroll
             for (int v = 0; v < V; ++v)
-                oh[v] = S ? f32_cell<SQ, true>(ch[v], L[v], R[v], uh[v], dh[v], S[v], p.f)
-                          : f32_cell<SQ, false>(ch[v], L[v], R[v], uh[v], dh[v], 0.0f, p.f);
+                oh[v] = f32_cell<SQ, true>(ch[v], L[v], R[v], uh[v], dh[v], S[v], p.f);
         } else {
             const float Lh0 = __shfl_up_sync(0xffffffffu, ch[V - 1], 1);
             const float Ll0 = __shfl_up_sync(0xffffffffu, cl[V - 1], 1);
@@ -360,7 +432,89 @@ struct FkStrip {
 #pragma unroll
             for (int v = 0; v < V; ++v)
                 fk_cell<SQ>(ch[v], cl[v], Lh[v], Ll[v], Rh[v], Rl[v], uh[v], ul[v], dh[v],
-                            dl[v], S ? S[v] : 0.0f, p.f, oh[v], ol[v]);
+                            dl[v], S[v], p.f, oh[v], ol[v]);
+        }
+    }
+
+    // One row of level T from the packed rows of level T-1 (interior and
+    // mirror-edge lanes): the scalar cell functions' operations in their
+    // order, two cells per instruction.
+    __device__ __forceinline__ void fast_update(const p2* uh, const p2* ul, const p2* ch,
+                                                const p2* cl, const p2* dh, const p2* dl,
+                                                p2* oh, p2* ol) {
+        const FkCoef2& f = p.f2;
+        const float h0 = p2_a(ch[0]), h1 = p2_b(ch[0]), h2 = p2_a(ch[1]), h3 = p2_b(ch[1]);
+        float Lo = __shfl_up_sync(0xffffffffu, h3, 1);
+        float Ro = __shfl_down_sync(0xffffffffu, h0, 1);
+        Lo = first_col ? h0 : Lo;
+        Ro = last_col ? h3 : Ro;
+        if constexpr (!COMP) {
+            const p2 rl[2] = {p2_pack(__fadd_rn(h1, Lo), __fadd_rn(h2, h0)),
+                              p2_pack(__fadd_rn(h3, h1), __fadd_rn(Ro, h2))};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const p2 t = ch[q];
+                const p2 t2 = p2_mul(t, t);
+                const p2 e4 = p2_fma(t2, t2, f.nTa4);
+                const p2 nloss = p2_fma(f.ncrad, e4, p2_fma(f.ncls, t, f.clsTa));
+                p2 net;
+                if constexpr (SQ) {
+                    const p2 lap = p2_fma(f.m4, t, p2_add(rl[q], p2_add(uh[q], dh[q])));
+                    net = p2_fma(f.ax, lap, nloss);
+                } else {
+                    const p2 lx = p2_fma(f.m2, t, rl[q]);
+                    const p2 ly = p2_fma(f.m2, t, p2_add(uh[q], dh[q]));
+                    net = p2_fma(f.ax, lx, p2_fma(f.ay, ly, nloss));
+                }
+                oh[q] = p2_add(t, net);
+            }
+        } else {
+            const float l0 = p2_a(cl[0]), l1 = p2_b(cl[0]), l2 = p2_a(cl[1]), l3 = p2_b(cl[1]);
+            float Ll = __shfl_up_sync(0xffffffffu, l3, 1);
+            float Rl = __shfl_down_sync(0xffffffffu, l0, 1);
+            Ll = first_col ? l0 : Ll;
+            Rl = last_col ? l3 : Rl;
+            // differences across the lane's faces: a cell's left difference is
+            // its left neighbour's right one, negated
+            const float a0 = __fsub_rn(h0, Lo), a1 = __fsub_rn(h1, h0), a2 = __fsub_rn(h2, h1),
+                        a3 = __fsub_rn(h3, h2), a4 = __fsub_rn(Ro, h3);
+            const p2 hx[2] = {p2_pack(__fsub_rn(a1, a0), __fsub_rn(a2, a1)),
+                              p2_pack(__fsub_rn(a3, a2), __fsub_rn(a4, a3))};
+            p2 lx[2];
+            if constexpr (SQ) {
+                lx[0] = p2_pack(__fadd_rn(l1, Ll), __fadd_rn(l2, l0));
+                lx[1] = p2_pack(__fadd_rn(l3, l1), __fadd_rn(Rl, l2));
+            } else {
+                const float b0 = __fsub_rn(l0, Ll), b1 = __fsub_rn(l1, l0), b2 = __fsub_rn(l2, l1),
+                            b3 = __fsub_rn(l3, l2), b4 = __fsub_rn(Rl, l3);
+                lx[0] = p2_pack(__fsub_rn(b1, b0), __fsub_rn(b2, b1));
+                lx[1] = p2_pack(__fsub_rn(b3, b2), __fsub_rn(b4, b3));
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const p2 th = ch[q], tl = cl[q];
+                const p2 da = p2_add(p2_sub(th, f.Ta_hi), p2_sub(tl, f.Ta_lo));
+                const p2 t = p2_add(th, tl);
+                const p2 t2 = p2_mul(t, t);
+                const p2 e4 = p2_fma(t2, t2, f.nTa4);
+                const p2 nloss = p2_fma(f.ncrad, e4, p2_mul(f.ncls, da));
+                const p2 hy = p2_add(p2_sub(dh[q], th), p2_sub(uh[q], th));
+                p2 d;
+                if constexpr (SQ) {
+                    const p2 lh = p2_add(hx[q], hy);
+                    const p2 ll = p2_fma(f.m4, tl, p2_add(lx[q], p2_add(dl[q], ul[q])));
+                    d = p2_fma(f.ax, p2_add(lh, ll), nloss);
+                } else {
+                    const p2 dx = p2_add(hx[q], lx[q]);
+                    const p2 dy = p2_add(hy, p2_add(p2_sub(dl[q], tl), p2_sub(ul[q], tl)));
+                    d = p2_fma(f.ax, dx, p2_fma(f.ay, dy, nloss));
+                }
+                const p2 sum = p2_add(th, d);
+                const p2 err = p2_sub(d, p2_sub(sum, th));
+                const p2 lo = p2_add(tl, err);
+                oh[q] = p2_add(sum, lo);
+                ol[q] = p2_sub(lo, p2_sub(oh[q], sum));
+            }
         }
     }
 
@@ -374,13 +528,39 @@ struct FkStrip {
     __device__ __forceinline__ void fast_level(int jj) {
         if constexpr (T <= K) {
             constexpr int su = mod3(P - T - 1), sc = mod3(P - T), sd = mod3(P - T + 1);
-            float (&ah)[3][V] = winh<T - 1>();
-            float (&al)[3][V] = winl<T - 1>();
-            float oh[V], ol[V];
-            row_update(ah[su], al[su], ah[sc], al[sc], ah[sd], al[sd], nullptr, oh, ol);
+            p2 (&ah)[3][2] = winh<T - 1>();
+            p2 (&al)[3][2] = winl<T - 1>();
+            p2 oh[2], ol[2];
+            fast_update(ah[su], al[su], ah[sc], al[sc], ah[sd], al[sd], oh, ol);
             const int r = jj - T;
-            const bool owned_row = r >= y0 && r < y1;
-            finish_level<T, sc>(r, oh, ol, owned_row, true);
+            const bool own = own_all && r >= y0 && r < y1;
+            if constexpr (T < K) {
+                p2 (&bh)[3][2] = winh<T>();
+                bh[sc][0] = oh[0]; bh[sc][1] = oh[1];
+                if constexpr (COMP) {
+                    p2 (&bl)[3][2] = winl<T>();
+                    bl[sc][0] = ol[0]; bl[sc][1] = ol[1];
+                }
+            } else {
+                const size_t off = (size_t)r * p.c.nx + xl;
+                st_global_v2_pred(p.Thi_out + off, oh, own);
+                if constexpr (COMP) st_global_v2_pred(p.Tlo_out + off, ol, own);
+            }
+            if constexpr (REDUCE) {
+                // the largest of the four cells against the box threshold (NaN
+                // never wins a maximum); pairs by the sign of their exact
+                // difference
+                const float th = own ? thr_h[T - 1] : INFINITY;
+                if constexpr (COMP) {
+                    const p2 tp = p2_pack(th, th), tq = p2_pack(thr_l[T - 1], thr_l[T - 1]);
+                    const p2 e0 = p2_add(p2_sub(oh[0], tp), p2_sub(ol[0], tq));
+                    const p2 e1 = p2_add(p2_sub(oh[1], tp), p2_sub(ol[1], tq));
+                    hit[T - 1] |= fmaxf(fmaxf(p2_a(e0), p2_b(e0)), fmaxf(p2_a(e1), p2_b(e1))) > 0.0f;
+                } else {
+                    hit[T - 1] |= fmaxf(fmaxf(p2_a(oh[0]), p2_b(oh[0])),
+                                        fmaxf(p2_a(oh[1]), p2_b(oh[1]))) > th;
+                }
+            }
             fast_level<P, T + 1>(jj);
         }
     }
@@ -401,20 +581,17 @@ struct FkStrip {
             const int lo = max(y0 - K + T, 0);
             const int hi = min(y1 - 1 + K - T, ny - 1);
             if (r >= lo && r <= hi) {
-                float (&ah)[3][V] = winh<T - 1>();
-                float (&al)[3][V] = winl<T - 1>();
-                if (r == 0) {
+                p2 (&ah)[3][2] = winh<T - 1>();
+                p2 (&al)[3][2] = winl<T - 1>();
 #pragma unroll
-                    for (int v = 0; v < V; ++v) {
-                        ah[su][v] = ah[sc][v];
-                        if constexpr (COMP) al[su][v] = al[sc][v];
+                for (int q = 0; q < 2; ++q) {
+                    if (r == 0) {
+                        ah[su][q] = ah[sc][q];
+                        if constexpr (COMP) al[su][q] = al[sc][q];
                     }
-                }
-                if (r == ny - 1) {
-#pragma unroll
-                    for (int v = 0; v < V; ++v) {
-                        ah[sd][v] = ah[sc][v];
-                        if constexpr (COMP) al[sd][v] = al[sc][v];
+                    if (r == ny - 1) {
+                        ah[sd][q] = ah[sc][q];
+                        if constexpr (COMP) al[sd][q] = al[sc][q];
                     }
                 }
                 float oh[V], ol[V];
@@ -429,7 +606,16 @@ struct FkStrip {
                         for (int v = 0; v < V; ++v)
                             S[v] = (float)src_product(rf, colf[(T - 1) * V + v]);
                     }
-                    row_update(ah[su], al[su], ah[sc], al[sc], ah[sd], al[sd], S, oh, ol);
+                    float uh[V], ul[V], ch[V], cl[V], dh[V], dl[V];
+                    unpack(ah[su], uh);
+                    unpack(ah[sc], ch);
+                    unpack(ah[sd], dh);
+                    if constexpr (COMP) {
+                        unpack(al[su], ul);
+                        unpack(al[sc], cl);
+                        unpack(al[sd], dl);
+                    }
+                    row_update(uh, ul, ch, cl, dh, dl, S, oh, ol);
                     if (edge && p.c.bc == 1) {
 #pragma unroll
                         for (int v = 0; v < V; ++v)
@@ -450,12 +636,13 @@ struct FkStrip {
     __device__ __forceinline__ void finish_level(int r, const float* oh, const float* ol,
                                                  bool owned_row, bool full) {
         if constexpr (T < K) {
-            float (&bh)[3][V] = winh<T>();
-            float (&bl)[3][V] = winl<T>();
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                bh[SC][v] = oh[v];
-                if constexpr (COMP) bl[SC][v] = ol[v];
+            p2 (&bh)[3][2] = winh<T>();
+            bh[SC][0] = p2_pack(oh[0], oh[1]);
+            bh[SC][1] = p2_pack(oh[2], oh[3]);
+            if constexpr (COMP) {
+                p2 (&bl)[3][2] = winl<T>();
+                bl[SC][0] = p2_pack(ol[0], ol[1]);
+                bl[SC][1] = p2_pack(ol[2], ol[3]);
             }
         } else {
             // nx is a multiple of 4 (checked on entry): an owned lane's four
@@ -507,16 +694,14 @@ struct FkStrip {
         if constexpr (T >= 1 && T < K) {
 #pragma unroll
             for (int P = 0; P < 3; ++P) {
-                constexpr int dummy = 0;
-                (void)dummy;
-                const int s = ((P - T) % 3 + 3) % 3;
-                float* d = s_box[P][lane];
+                const int sl = ((P - T) % 3 + 3) % 3;
+                p2* d = reinterpret_cast<p2*>(s_box[P][lane]);
 #pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    d[v] = (s == 0) ? winh<T>()[0][v] : (s == 1) ? winh<T>()[1][v] : winh<T>()[2][v];
+                for (int q = 0; q < 2; ++q) {
+                    d[q] = (sl == 0) ? winh<T>()[0][q] : (sl == 1) ? winh<T>()[1][q] : winh<T>()[2][q];
                     if constexpr (COMP)
-                        d[V + v] = (s == 0) ? winl<T>()[0][v]
-                                 : (s == 1) ? winl<T>()[1][v] : winl<T>()[2][v];
+                        d[2 + q] = (sl == 0) ? winl<T>()[0][q]
+                                 : (sl == 1) ? winl<T>()[1][q] : winl<T>()[2][q];
                 }
             }
         }
@@ -587,8 +772,13 @@ struct FkStrip {
     }
 };
 
+// Resident CTAs per SM the register budget is sized for: the plain field's
+// 24 KB of stages admit more than three.
+template <int K, bool COMP>
+struct FkOcc { static constexpr int min_ctas = !COMP && K <= 3 ? 4 : 3; };
+
 template <int K, bool REDUCE, bool SQ, bool COMP>
-__global__ void __launch_bounds__(ADV_WARPS * 32, AdvOcc<K>::min_ctas)
+__global__ void __launch_bounds__(ADV_WARPS * 32, FkOcc<K, COMP>::min_ctas)
 advance_f32k_kernel(const __grid_constant__ CUtensorMap map_hi,
                     const __grid_constant__ CUtensorMap map_lo,
                     const __grid_constant__ FkParams p) {
