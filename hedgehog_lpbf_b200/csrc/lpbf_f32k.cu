@@ -69,10 +69,17 @@ cudaError_t launch_fk(const float* hi_in, const float* lo_in, float* hi_out, flo
     p.nstrips = (c.nx + ADV_WOUT - 1) / ADV_WOUT;
     int H = rows;
     if (H <= 0) {
-        // about three tasks per resident warp, 12..48 rows (48 measured best
-        // at 8192^2, depth 3, for both fields over the bench raster)
-        const long long want = (long long)c.ny * p.nstrips / (3ll * resident * ADV_WARPS);
-        H = (int)std::max(12ll, std::min(48ll, want));
+        // 12..64 rows with the fewest waves x rows a task computes, as for the
+        // FP64 field (4096^2, depth 3, us per step: plain 21.4 with 62 rows
+        // against 26.5 with three tasks per warp; compensated 54.6 with 41
+        // against 61.4)
+        const long long warps = (long long)resident * ADV_WARPS;
+        long long best = -1;
+        for (int h = 12; h <= 64; ++h) {
+            const long long tasks = (long long)((c.ny + h - 1) / h) * p.nstrips;
+            const long long cost = ((tasks + warps - 1) / warps) * (h + 2 * K);
+            if (best < 0 || cost <= best) { best = cost; H = h; }
+        }
     }
     p.H = std::max(std::min(H, c.ny), 1);
     // rows whose tasks (owned rows +- K) reach the source band: 8-row tasks
@@ -203,11 +210,9 @@ int lpbf_b200_advance_f32k(float* hi_a, float* lo_a, float* hi_b, float* lo_b,
     Workspace* ws = static_cast<Workspace*>(work);
     if (!ws || work_bytes < sizeof(Workspace)) return LPBF_ERR_WORKSPACE;
 
-    int depth = opts->depth;
-    if (depth <= 0) {
-        const long long n = (long long)N;
-        depth = (n >= (1ll << 22)) ? 3 : (n >= (1ll << 18)) ? 2 : 1;
-    }
+    // Measured on B200 (us per step): 128^2 17.0, 12.0, 12.0, 13.2 at depths
+    // 1-4; 4096^2 depth 2 53.9, 3 51.6, 4 60.8 (depth 4 spills).
+    int depth = opts->depth > 0 ? opts->depth : 3;
     depth = std::min(std::max(depth, 1), 4);
     const Coef c = make_coef(*k, opts->bc, opts->T_edge, opts->Tm);
     const FkCoef f = make_fk(c, opts->T_edge);
@@ -247,11 +252,9 @@ int lpbf_b200_advance_f32(float* T_a, float* T_b, const StepConst* k, const lpbf
     Workspace* ws = static_cast<Workspace*>(work);
     if (!ws || work_bytes < sizeof(Workspace)) return LPBF_ERR_WORKSPACE;
 
-    int depth = opts->depth;
-    if (depth <= 0) {
-        const long long n = (long long)N;
-        depth = (n >= (1ll << 22)) ? 3 : (n >= (1ll << 18)) ? 2 : 1;
-    }
+    // Measured on B200 (us per step): 128^2 15.0, 10.8, 10.2, 9.0 at depths
+    // 1-4; 8192^2 depth 2 63.5, 3 56.8, 4 53.2.
+    int depth = opts->depth > 0 ? opts->depth : 4;
     depth = std::min(std::max(depth, 1), 4);
     const Coef c = make_coef(*k, opts->bc, opts->T_edge, opts->Tm);
     const FkCoef f = make_fk(c, opts->T_edge);

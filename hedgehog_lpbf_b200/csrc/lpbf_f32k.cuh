@@ -43,14 +43,12 @@ constexpr size_t fk_smem_bytes() {
            + size_t(ADV_WARPS) * ADV_S * sizeof(uint64_t);
 }
 
-// 16-byte store issued under a predicate (no branch).  It carries a
-// "memory" clobber: the exact reduction reads level-K values back from the
-// output field, and those loads must stay after the stores.
+// 16-byte store issued under a predicate (no branch), without a "memory"
+// clobber: the kernel never reads the destination field back.
 __device__ __forceinline__ void st_global_v4f_pred(float* p, const float* v, bool pred) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
                  "@q st.global.v4.f32 [%0], {%1, %2, %3, %4};\n\t}"
-                 :: "l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"((int)pred)
-                 : "memory");
+                 :: "l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"((int)pred));
 }
 
 // ---- packed pairs of f32 -----------------------------------------------------
@@ -111,8 +109,7 @@ struct FkCoef2 {
 __device__ __forceinline__ void st_global_v2_pred(float* p, const p2* v, bool pred) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\t"
                  "@q st.global.v2.b64 [%0], {%1, %2};\n\t}"
-                 :: "l"(p), "l"(v[0]), "l"(v[1]), "r"((int)pred)
-                 : "memory");
+                 :: "l"(p), "l"(v[0]), "l"(v[1]), "r"((int)pred));
 }
 
 struct FkCoef {
@@ -235,6 +232,7 @@ struct FkStrip {
     p2 wh[K > 1 ? K - 1 : 1][3][2], wl[K > 1 ? K - 1 : 1][3][2];
     float thr_h[K], thr_l[K];
     bool hit[K];
+    unsigned kmask;                    // last-level rows of this box in s_box
     double (*s_tmx)[32];
     long long (*s_arg)[32];
     int* s_ymn;
@@ -245,7 +243,7 @@ struct FkStrip {
                                        const CUtensorMap* ml, float* st, uint64_t* b, int ln,
                                        double (*tm)[32], long long (*ar)[32], int* mn, int* mx,
                                        float (*bx)[32][2 * ADV_V])
-        : p(p_), map_hi(mh), map_lo(ml), stages(st), bars(b), gbox(0), lane(ln), failed(false),
+        : p(p_), map_hi(mh), map_lo(ml), stages(st), bars(b), gbox(0), lane(ln), failed(false), kmask(0u),
           s_tmx(tm), s_arg(ar), s_ymn(mn), s_ymx(mx), s_box(bx) {
         if constexpr (REDUCE) {
             const long long N = (long long)p.c.nx * p.c.ny;
@@ -337,16 +335,20 @@ struct FkStrip {
             // outer neighbours itself (nx a multiple of 4: whole lanes)
             const bool src_box = src_strip && j + 1 >= p.band_lo && j - K <= p.band_hi;
             const bool fast = (!edge || (p.c.bc == 0 && (p.c.nx & 3) == 0)) &&
-                              j - K >= 1 && j + 1 <= ny - 2 && !src_box;
+                              j - K >= 1 && j + 1 <= ny - 2 && j < jend;
             rowf = 0.0;
             if (src_box) {
                 const int t = min(lane / 3, K - 1);
                 rowf = src_row(j + lane % 3 - (t + 1), p.las[t], p.c);
             }
-            if (fast && j < jend) {
-                fast_row<0>(j, st);
-                fast_row<1>(j + 1, st);
-                fast_row<2>(j + 2, st);
+            if (fast && !src_box) {
+                fast_row<0, false>(j, st);
+                fast_row<1, false>(j + 1, st);
+                fast_row<2, false>(j + 2, st);
+            } else if (fast) {
+                fast_row<0, true>(j, st);
+                fast_row<1, true>(j + 1, st);
+                fast_row<2, true>(j + 2, st);
             } else {
                 general_row<0>(j, st, jlast);
                 general_row<1>(j + 1, st, jlast);
@@ -438,10 +440,11 @@ struct FkStrip {
 
     // One row of level T from the packed rows of level T-1 (interior and
     // mirror-edge lanes): the scalar cell functions' operations in their
-    // order, two cells per instruction.
+    // order, two cells per instruction.  SRC: with the source increments S.
+    template <bool SRC>
     __device__ __forceinline__ void fast_update(const p2* uh, const p2* ul, const p2* ch,
                                                 const p2* cl, const p2* dh, const p2* dl,
-                                                p2* oh, p2* ol) {
+                                                const p2* S, p2* oh, p2* ol) {
         const FkCoef2& f = p.f2;
         const float h0 = p2_a(ch[0]), h1 = p2_b(ch[0]), h2 = p2_a(ch[1]), h3 = p2_b(ch[1]);
         float Lo = __shfl_up_sync(0xffffffffu, h3, 1);
@@ -466,6 +469,7 @@ struct FkStrip {
                     const p2 ly = p2_fma(f.m2, t, p2_add(uh[q], dh[q]));
                     net = p2_fma(f.ax, lx, p2_fma(f.ay, ly, nloss));
                 }
+                if constexpr (SRC) net = p2_add(net, S[q]);
                 oh[q] = p2_add(t, net);
             }
         } else {
@@ -497,7 +501,8 @@ struct FkStrip {
                 const p2 t = p2_add(th, tl);
                 const p2 t2 = p2_mul(t, t);
                 const p2 e4 = p2_fma(t2, t2, f.nTa4);
-                const p2 nloss = p2_fma(f.ncrad, e4, p2_mul(f.ncls, da));
+                p2 nloss = p2_fma(f.ncrad, e4, p2_mul(f.ncls, da));
+                if constexpr (SRC) nloss = p2_add(S[q], nloss);
                 const p2 hy = p2_add(p2_sub(dh[q], th), p2_sub(uh[q], th));
                 p2 d;
                 if constexpr (SQ) {
@@ -518,20 +523,27 @@ struct FkStrip {
         }
     }
 
-    template <int P>
+    template <int P, bool SRC>
     __device__ __forceinline__ void fast_row(int jj, const float* st) {
         load_row0<P>(st);
-        fast_level<P, 1>(jj);
+        fast_level<P, 1, SRC>(jj);
     }
 
-    template <int P, int T>
+    template <int P, int T, bool SRC>
     __device__ __forceinline__ void fast_level(int jj) {
         if constexpr (T <= K) {
             constexpr int su = mod3(P - T - 1), sc = mod3(P - T), sd = mod3(P - T + 1);
             p2 (&ah)[3][2] = winh<T - 1>();
             p2 (&al)[3][2] = winl<T - 1>();
-            p2 oh[2], ol[2];
-            fast_update(ah[su], al[su], ah[sc], al[sc], ah[sd], al[sd], oh, ol);
+            p2 oh[2], ol[2], S[2];
+            if constexpr (SRC) {
+                __syncwarp();              // bounds the interleaving of levels (registers)
+                const double rf = __shfl_sync(0xffffffffu, rowf, 3 * (T - 1) + P);
+                const double* cf = colf + (T - 1) * V;
+                S[0] = p2_pack((float)src_product(rf, cf[0]), (float)src_product(rf, cf[1]));
+                S[1] = p2_pack((float)src_product(rf, cf[2]), (float)src_product(rf, cf[3]));
+            }
+            fast_update<SRC>(ah[su], al[su], ah[sc], al[sc], ah[sd], al[sd], S, oh, ol);
             const int r = jj - T;
             const bool own = own_all && r >= y0 && r < y1;
             if constexpr (T < K) {
@@ -551,17 +563,22 @@ struct FkStrip {
                 // never wins a maximum); pairs by the sign of their exact
                 // difference
                 const float th = own ? thr_h[T - 1] : INFINITY;
+                bool rh;
                 if constexpr (COMP) {
                     const p2 tp = p2_pack(th, th), tq = p2_pack(thr_l[T - 1], thr_l[T - 1]);
                     const p2 e0 = p2_add(p2_sub(oh[0], tp), p2_sub(ol[0], tq));
                     const p2 e1 = p2_add(p2_sub(oh[1], tp), p2_sub(ol[1], tq));
-                    hit[T - 1] |= fmaxf(fmaxf(p2_a(e0), p2_b(e0)), fmaxf(p2_a(e1), p2_b(e1))) > 0.0f;
+                    rh = fmaxf(fmaxf(p2_a(e0), p2_b(e0)), fmaxf(p2_a(e1), p2_b(e1))) > 0.0f;
                 } else {
-                    hit[T - 1] |= fmaxf(fmaxf(p2_a(oh[0]), p2_b(oh[0])),
-                                        fmaxf(p2_a(oh[1]), p2_b(oh[1]))) > th;
+                    rh = fmaxf(fmaxf(p2_a(oh[0]), p2_b(oh[0])),
+                               fmaxf(p2_a(oh[1]), p2_b(oh[1]))) > th;
+                }
+                hit[T - 1] |= rh;
+                if constexpr (T == K) {
+                    if (rh) stage_row<P>(oh, ol);
                 }
             }
-            fast_level<P, T + 1>(jj);
+            fast_level<P, T + 1, SRC>(jj);
         }
     }
 
@@ -624,7 +641,7 @@ struct FkStrip {
                             }
                     }
                 }
-                finish_level<T, sc>(r, oh, ol, r >= y0 && r < y1, !edge);
+                finish_level<P, T, sc>(r, oh, ol, r >= y0 && r < y1, !edge);
             }
             general_level<P, T + 1>(jj);
         }
@@ -632,7 +649,7 @@ struct FkStrip {
 
     // Keep the new row in level T's window slot SC (T < K) or store it
     // (T == K), and test it against the box threshold.
-    template <int T, int SC>
+    template <int P, int T, int SC>
     __device__ __forceinline__ void finish_level(int r, const float* oh, const float* ol,
                                                  bool owned_row, bool full) {
         if constexpr (T < K) {
@@ -654,7 +671,7 @@ struct FkStrip {
             if constexpr (COMP) st_global_v4f_pred(p.Tlo_out + off, ol, st);
         }
         if constexpr (REDUCE) {
-            bool h = hit[T - 1];
+            bool h = false;
             const bool ol_ok = owned_row && owned_lane();
 #pragma unroll
             for (int v = 0; v < V; ++v) {
@@ -664,7 +681,18 @@ struct FkStrip {
                 else
                     h = h | (ok && oh[v] > thr_h[T - 1]);
             }
-            hit[T - 1] = h;
+            hit[T - 1] |= h;
+            if constexpr (T == K) {
+                if (h) {
+                    const p2 ph[2] = {p2_pack(oh[0], oh[1]), p2_pack(oh[2], oh[3])};
+                    p2 pl[2] = {0ull, 0ull};
+                    if constexpr (COMP) {
+                        pl[0] = p2_pack(ol[0], ol[1]);
+                        pl[1] = p2_pack(ol[2], ol[3]);
+                    }
+                    stage_row<P>(ph, pl);
+                }
+            }
         }
     }
 
@@ -707,46 +735,66 @@ struct FkStrip {
         }
     }
 
-    __device__ __forceinline__ double value_at(int t, int P, int r, int v) const {
-        const size_t off = (size_t)r * p.c.nx + xl + v;
+    // A last-level row that crossed its threshold (box row P), for the exact
+    // pass: the last level has no register window, and reading the stored
+    // row back costs an L2 round trip per box.
+    template <int P>
+    __device__ __forceinline__ void stage_row(const p2* h, const p2* l) {
+        p2* d = reinterpret_cast<p2*>(s_box[P][lane]);
+        d[0] = h[0];
+        d[1] = h[1];
         if constexpr (COMP) {
-            if (t < K) return (double)s_box[P][lane][v] + (double)s_box[P][lane][V + v];
-            return (double)p.Thi_out[off] + (double)p.Tlo_out[off];
-        } else {
-            if (t < K) return (double)s_box[P][lane][v];
-            return (double)p.Thi_out[off];
+            d[2] = l[0];
+            d[3] = l[1];
         }
+        kmask |= 1u << P;
     }
 
-    __device__ __forceinline__ void exact_level(int t, int j) {
+    // Exact update of level t from the lane's rows in s_box (those of `rows`):
+    // its first maximal owned cell in flat-index order and the molten rows.
+    __device__ __forceinline__ void exact_level(int t, int j, unsigned rows) {
         const int nx = p.c.nx;
-        const bool ol = owned_lane();
+        unsigned molten = 0u;
         double m = -INFINITY;
+        int a = -1;
+#pragma unroll
         for (int P = 0; P < 3; ++P) {
             const int r = j + P - t;
-            const bool cand = r >= y0 && r < y1 && ol;
-            bool hot = false;
+            const bool cand = ((rows >> P) & 1u) && r >= y0 && r < y1 && own_all;
+            const float4 h = *reinterpret_cast<const float4*>(&s_box[P][lane][0]);
+            const float hv[V] = {h.x, h.y, h.z, h.w};
+            double c[V];
+            if constexpr (COMP) {
+                const float4 l = *reinterpret_cast<const float4*>(&s_box[P][lane][V]);
+                const float lv[V] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+                for (int v = 0; v < V; ++v) c[v] = (double)hv[v] + (double)lv[v];
+            } else {
+#pragma unroll
+                for (int v = 0; v < V; ++v) c[v] = (double)hv[v];
+            }
+#pragma unroll
             for (int v = 0; v < V; ++v) {
-                const bool ok = cand && xl + v < nx;
-                const double x = ok ? value_at(t, P, r, v) : 0.0;
-                m = (ok && x > m) ? x : m;
-                hot |= ok && x > p.c.Tm;
+                molten |= cand && c[v] > p.c.Tm ? 1u << P : 0u;
+                c[v] = cand && c[v] > -INFINITY ? c[v] : -INFINITY;      // NaN never wins
             }
-            if (__any_sync(0xffffffffu, hot) && lane == 0) {
-                s_ymn[t - 1] = min(s_ymn[t - 1], r);
-                s_ymx[t - 1] = max(s_ymx[t - 1], r);
-            }
+            // pairs, then their winners (strict '>': the smaller index)
+            const bool h01 = c[1] > c[0], h23 = c[3] > c[2];
+            const double m01 = h01 ? c[1] : c[0], m23 = h23 ? c[3] : c[2];
+            const bool hh = m23 > m01;
+            const double mr = hh ? m23 : m01;
+            const int ar = P * V + (hh ? (h23 ? 3 : 2) : (h01 ? 1 : 0));
+            a = mr > m ? ar : a;
+            m = mr > m ? mr : m;
+        }
+        molten = __reduce_or_sync(0xffffffffu, molten);
+        if (molten && lane == 0) {
+            s_ymn[t - 1] = min(s_ymn[t - 1], j - t + __ffs(molten) - 1);
+            s_ymx[t - 1] = max(s_ymx[t - 1], j - t + 31 - __clz(molten));
         }
         if (m > s_tmx[t - 1][lane]) {
-            long long arg = -1;
-            for (int P = 0; P < 3 && arg < 0; ++P) {
-                const int r = j + P - t;
-                if (!(r >= y0 && r < y1 && ol)) continue;
-                for (int v = 0; v < V && xl + v < nx; ++v)
-                    if (value_at(t, P, r, v) == m) { arg = (long long)r * nx + xl + v; break; }
-            }
             s_tmx[t - 1][lane] = m;
-            s_arg[t - 1][lane] = arg;
+            s_arg[t - 1][lane] = (long long)(j + a / V - t) * nx + xl + a % V;
         }
     }
 
@@ -756,18 +804,21 @@ struct FkStrip {
         for (int t = 0; t < K; ++t) { bits |= hit[t] ? (1u << t) : 0u; hit[t] = false; }
         bits = __reduce_or_sync(0xffffffffu, bits);
         if (bits == 0u) return;
-        for (int t = 1; t <= K; ++t) {
+        // the last level first: its rows sit in s_box, where the others are
+        // staged from their windows in turn (a lane reads only its own)
+#pragma unroll 1
+        for (int t = K; t >= 1; --t) {
             if (!((bits >> (t - 1)) & 1u)) continue;
-            switch (t) {
+            switch (t < K ? t : 0) {
                 case 1: stage_level<1>(); break;
                 case 2: stage_level<2>(); break;
                 case 3: stage_level<3>(); break;
                 default: break;
             }
-            __syncwarp();
-            exact_level(t, j);
-            __syncwarp();
+            exact_level(t, j, t < K ? 7u : kmask);
         }
+        kmask = 0u;
+        __syncwarp();
         set_thresholds();
     }
 };
