@@ -123,9 +123,9 @@ inline cudaError_t launch_finalize(const Partial* parts, int nblocks, int nx, in
 
 constexpr int EXT_WARPS = 8;       // warps per CTA
 constexpr int EXT_V = 2;           // columns per lane
-constexpr int EXT_OWN = 32 * EXT_V - 2;   // columns a warp owns (the first and last are halo)
-constexpr int EXT_H = 64;          // rows per task
-constexpr int EXT_PF = 8;          // rows loaded ahead of the one being updated
+constexpr int EXT_OWN = 30 * EXT_V;   // columns a warp owns (its first and last lane are halo)
+constexpr int EXT_H = 64;          // most rows per task
+constexpr int EXT_R = 4;           // rows per block: updated together, the next block's loaded ahead
 
 struct ExtParams {
     StepConst k;
@@ -135,7 +135,7 @@ struct ExtParams {
     double dt_rho;                 // dt / rho
     double r2_cut;                 // beyond this r^2 the source is below 2^-80 of its peak
     int band_lo, band_hi, bandx_lo, bandx_hi;   // cells the source can reach
-    int nstrips, ntasks;
+    int nstrips, H, ntasks;
     int bc;
     double T_edge, Tm;
     Partial* ring;
@@ -157,16 +157,15 @@ __device__ __forceinline__ double rcp_newton(double d) {
     return fma(r, e, r);
 }
 
-// The laser's heat input q_in at cell (x, y) (kernels.cu:141 order), zero
-// where r^2 >= r2_cut (below 2^-80 of the peak).  Out of line: the exp code
+// One factor of the laser's heat input (kernels.cu:141): the input is a row
+// factor (with the amplitude) times a column factor, each zero beyond the
+// truncation radius, as in the baseline kernel.  Out of line: the exp code
 // exists once in the binary and holds no registers in the row loop.
-static __device__ __noinline__ double ext_source(int x, int y, const StepConst& k,
-                                                 double r2_cut) {
-    const double xd = __dsub_rn(__dmul_rn((double)x, k.dx), k.x_l);
-    const double yd = __dsub_rn(__dmul_rn((double)y, k.dy), k.y_l);
-    const double r2 = __dadd_rn(__dmul_rn(xd, xd), __dmul_rn(yd, yd));
-    if (r2 >= r2_cut) return 0.0;
-    return k.q_scale * k.peak_S * exp(__dmul_rn(-2.0 * r2, k.inv_r0_sq));
+static __device__ __noinline__ double ext_factor(int i, double d, double centre,
+                                                 double inv_r0_sq, double r2_cut) {
+    const double z = __dsub_rn(__dmul_rn((double)i, d), centre);
+    const double z2 = __dmul_rn(z, z);
+    return z2 < r2_cut ? exp(__dmul_rn(-2.0 * z2, inv_r0_sq)) : 0.0;
 }
 
 // The ordering key of T (see ExtLines).
@@ -203,17 +202,17 @@ __device__ __forceinline__ double ext_keff(double T, unsigned int key, int s, co
 }
 
 // A cell as the row stream carries it: T, k_eff(T), k_of(T) (the substrate
-// loss uses the conductivity without kmult), its ordering key and segment.
-struct ExtCell { double T, k, kp; unsigned int key; int seg; };
+// loss uses the conductivity without kmult) and its segment.
+struct ExtCell { double T, k, kp; int seg; };
 
 template <bool KM>
 __device__ __forceinline__ ExtCell ext_cell(double T, const ExtLines& L, const ExtLines& Lp,
                                             double kmult) {
     ExtCell c;
     c.T = T;
-    c.key = ext_key(T);
-    c.seg = ext_seg(c.key, L);
-    c.k = ext_keff<KM>(T, c.key, c.seg, L, Lp, kmult, c.kp);
+    const unsigned int key = ext_key(T);
+    c.seg = ext_seg(key, L);
+    c.k = ext_keff<KM>(T, key, c.seg, L, Lp, kmult, c.kp);
     return c;
 }
 
@@ -225,23 +224,164 @@ __device__ __forceinline__ double ext_flux(const ExtCell& a, const ExtCell& b) {
 }
 
 // The new temperature of cell c from div(k grad T) and the source:
-// T + dt (div + (q_in - q_top - q_bot) / h) / (rho cp_eff(T)).
+// T + dt (div + (q_in - q_top - q_bot) / h) / (rho cp_eff(T)).  With one
+// surrounding temperature (SAMET: Tamb == Tsub) convection and conduction
+// share their difference.
+template <bool SAMET, bool SRC>
 __device__ __forceinline__ double ext_update(const ExtCell& c, double div, double q_in,
                                              const StepConst& k, const ExtParams& p,
                                              const ExtLines& L) {
     const double T = c.T;
     const double T2 = __dmul_rn(T, T);
-    const double q_top = fma(p.esig, fma(T2, T2, -p.Ta4), k.hConv * (T - k.Tamb));
-    const double q_bot = __dmul_rn(c.kp * p.r_dsub, T - k.Tsub);
-    const double rhs = fma(q_in - (q_top + q_bot), k.inv_h, div);
+    const double e4 = fma(T2, T2, -p.Ta4);
+    const double da = __dsub_rn(T, k.Tamb);
+    double q;
+    if constexpr (SAMET)
+        q = fma(p.esig, e4, __dmul_rn(da, fma(c.kp, p.r_dsub, k.hConv)));
+    else
+        q = fma(p.esig, e4, fma(__dmul_rn(c.kp, p.r_dsub), __dsub_rn(T, k.Tsub),
+                                __dmul_rn(k.hConv, da)));
+    const double rhs = SRC ? fma(q_in - q, k.inv_h, div) : fma(-q, k.inv_h, div);
     double cp = fma(L.bc[c.seg], T, L.ac[c.seg]);
-    if (c.key >= p.L.sol_key && c.key <= p.L.liq_key) cp += LATENT * INV_MUSHY;
+    const unsigned int key = ext_key(T);
+    if (key >= p.L.sol_key && key <= p.L.liq_key) cp += LATENT * INV_MUSHY;
     return fma(__dmul_rn(rhs, p.dt_rho), rcp_newton(cp), T);
 }
 
-// One warp advances one (strip, chunk) task: 62 owned columns (lane l holds
-// the two columns xs + 2l and xs + 2l + 1; lane 0's first and lane 31's
-// second are the neighbours either side) down H rows.  Each cell's T and
+// A warp's place in the field and its carried rows: the centre row's cells and
+// the fluxes through the faces above them.
+struct ExtStrip {
+    int xa, xb, cv, ca, cb;        // the lane's columns; clamped load columns
+    bool own, own_b;
+    int y1;
+    ExtCell a, b;
+    double Fua, Fub;
+    double cfa, cfb;               // column factors of the source
+    double thr, tm;                // reduction: threshold, lane peak and its cell
+    int py, px, mn, mx;
+};
+
+// Row y (clamped to the field) of the lane's two columns.  VEC (rows on
+// 16-byte boundaries, nx even): a pair lies wholly on or off the field; one
+// off it takes the edge cell twice.
+template <bool VEC>
+__device__ __forceinline__ void ext_load(const double* __restrict__ Tin, int nx, int ny, int y,
+                                         const ExtStrip& s, double& u, double& v) {
+    const double* row = Tin + (size_t)min(max(y, 0), ny - 1) * nx;
+    if constexpr (VEC) {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(row + s.cv));
+        u = s.xa >= nx ? t.y : t.x;
+        v = s.xa < 0 ? t.x : t.y;
+    } else {
+        u = __ldg(row + s.ca);
+        v = __ldg(row + s.cb);
+    }
+}
+
+// EXT_R rows from y on (those below y1) in one straight line: their lower
+// neighbours' values in Q (replaced by the next block's), no branch between
+// rows, so the rows' chains (a table lookup is three dependent shared loads,
+// the reciprocal five dependent operations) overlap.  With a branch per row a
+// lone warp took 1 us per row.  SRC: the block meets the source.
+template <bool REDUCE, bool KM, bool SAMET, bool VEC, bool SRC>
+__device__ __forceinline__ void ext_block(const double* __restrict__ Tin,
+                                          double* __restrict__ Tout, const ExtParams& p,
+                                          const ExtLines& L, int y, ExtStrip& s,
+                                          double (&Q)[EXT_R][2], int lane) {
+    const StepConst& k = p.k;
+    const int nx = k.nx, ny = k.ny;
+    ExtCell da[EXT_R], db[EXT_R];
+#pragma unroll
+    for (int i = 0; i < EXT_R; ++i) {
+        da[i] = ext_cell<KM>(Q[i][0], L, p.L, k.kmult);
+        db[i] = ext_cell<KM>(Q[i][1], L, p.L, k.kmult);
+    }
+    // the next block's rows (past the task's end: a clamped, unused row)
+#pragma unroll
+    for (int i = 0; i < EXT_R; ++i)
+        ext_load<VEC>(Tin, nx, ny, y + EXT_R + 1 + i, s, Q[i][0], Q[i][1]);
+    // row factors of the source, one row per lane
+    double rfl = 0.0;
+    if constexpr (SRC) {
+        const double f = ext_factor(y + min(lane, EXT_R - 1), k.dy, k.y_l, k.inv_r0_sq, p.r2_cut);
+        rfl = f > 0.0 ? k.q_scale * k.peak_S * f : 0.0;
+    }
+    double va[EXT_R], vb[EXT_R];
+#pragma unroll
+    for (int i = 0; i < EXT_R; ++i) {
+        // x faces: a|b inside the lane, b|next lane's a, and the previous
+        // lane's b|a as this lane's left face; y faces: down, carried up
+        const double Fab = ext_flux(s.a, s.b);
+        const double TR = __shfl_down_sync(0xffffffffu, s.a.T, 1);
+        const double kR = __shfl_down_sync(0xffffffffu, s.a.k, 1);
+        const double FbR = __dmul_rn(__dadd_rn(s.b.k, kR), __dsub_rn(TR, s.b.T));
+        const double FLa = __shfl_up_sync(0xffffffffu, FbR, 1);
+        const double Fda = ext_flux(s.a, da[i]), Fdb = ext_flux(s.b, db[i]);
+        const double diva = fma(__dsub_rn(Fda, s.Fua), p.hy, __dmul_rn(__dsub_rn(Fab, FLa), p.hx));
+        const double divb = fma(__dsub_rn(Fdb, s.Fub), p.hy, __dmul_rn(__dsub_rn(FbR, Fab), p.hx));
+        double qa = 0.0, qb = 0.0;
+        if constexpr (SRC) {
+            const double rf = __shfl_sync(0xffffffffu, rfl, i);
+            qa = s.cfa > 0.0 ? __dmul_rn(rf, s.cfa) : 0.0;
+            qb = s.cfb > 0.0 ? __dmul_rn(rf, s.cfb) : 0.0;
+        }
+        va[i] = ext_update<SAMET, SRC>(s.a, diva, qa, k, p, L);
+        vb[i] = ext_update<SAMET, SRC>(s.b, divb, qb, k, p, L);
+        s.Fua = Fda; s.Fub = Fdb;
+        s.a = da[i]; s.b = db[i];
+    }
+    if (p.bc == 1) {
+#pragma unroll
+        for (int i = 0; i < EXT_R; ++i) {
+            const bool ey = y + i == 0 || y + i == ny - 1;
+            if (ey || s.xa == 0 || s.xa == nx - 1) va[i] = p.T_edge;
+            if (ey || s.xb == 0 || s.xb == nx - 1) vb[i] = p.T_edge;
+        }
+    }
+    double* row = Tout + (size_t)y * nx + s.xa;
+#pragma unroll
+    for (int i = 0; i < EXT_R; ++i) {
+        const bool in = y + i < s.y1;
+        if constexpr (VEC) {
+            asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\t"
+                         "@q st.global.v2.f64 [%0], {%1, %2};\n\t}"
+                         :: "l"(row + (size_t)i * nx), "d"(va[i]), "d"(vb[i]),
+                            "r"((int)(in && s.own)));
+        } else {
+            if (in && s.own) row[(size_t)i * nx] = va[i];
+            if (in && s.own_b) row[(size_t)i * nx + 1] = vb[i];
+        }
+    }
+    if constexpr (REDUCE) {
+        // tested against min(lane peak, Tm); only a block in which some lane
+        // crosses it updates peaks and molten rows.  A lane meets its cells in
+        // increasing index order (rows down, a before b): strict '>' keeps the
+        // first maximum; NaN never wins
+        bool hit = false;
+#pragma unroll
+        for (int i = 0; i < EXT_R; ++i) hit |= va[i] > s.thr || vb[i] > s.thr;
+        if (__any_sync(0xffffffffu, hit)) {
+            unsigned int rows = 0u;
+#pragma unroll
+            for (int i = 0; i < EXT_R; ++i) {
+                const bool ka = s.own && y + i < s.y1, kb = s.own_b && y + i < s.y1;
+                if (ka && va[i] > s.tm) { s.tm = va[i]; s.py = y + i; s.px = s.xa; }
+                if (kb && vb[i] > s.tm) { s.tm = vb[i]; s.py = y + i; s.px = s.xb; }
+                rows |= (ka && va[i] > p.Tm) || (kb && vb[i] > p.Tm) ? 1u << i : 0u;
+            }
+            rows = __reduce_or_sync(0xffffffffu, rows);
+            if (rows) {
+                s.mn = min(s.mn, y + __ffs(rows) - 1);
+                s.mx = max(s.mx, y + 31 - __clz(rows));
+            }
+            s.thr = s.own ? (s.tm < p.Tm ? s.tm : p.Tm) : INFINITY;
+        }
+    }
+}
+
+// One warp advances one (strip, chunk) task: 60 owned columns (lane l holds
+// the two columns xs + 2l and xs + 2l + 1; the outer lanes are the neighbours
+// either side) down H rows.  Each cell's T and
 // k_eff are loaded and evaluated once, when its row enters; a face's flux
 // (k_a + k_b)(T_b - T_a) is computed once, inside the lane, by the lane to
 // its left (passed on by a shuffle) or by the cell above it (y faces,
@@ -254,7 +394,7 @@ __device__ __forceinline__ double ext_update(const ExtCell& c, double div, doubl
 // T + dt rhs / (rho cp_eff(T)) with 1/cp_eff by rcp_newton.  Partials as in
 // the baseline kernel: per lane over its owned cells, then warps, CTAs and
 // the last CTA.
-template <bool REDUCE, bool KM>
+template <bool REDUCE, bool KM, bool SAMET, bool VEC>
 __global__ void __launch_bounds__(EXT_WARPS * 32, 2)
 ext_step_kernel(const double* __restrict__ Tin, double* __restrict__ Tout,
                 const __grid_constant__ ExtParams p) {
@@ -269,101 +409,59 @@ ext_step_kernel(const double* __restrict__ Tin, double* __restrict__ Tout,
     __syncthreads();
     const int nx = k.nx, ny = k.ny;
     const long long N = (long long)nx * ny;
-    const double kmult = k.kmult;
-
-    double tm = -1.0;
-    long long ag = N;
-    int mn = ny, mx = -1;
+    ExtStrip s;
+    s.tm = -1.0;
+    s.py = -1; s.px = 0;                   // no peak cell yet
+    s.mn = ny; s.mx = -1;
     for (int task = blockIdx.x * EXT_WARPS + wid; task < p.ntasks;
          task += gridDim.x * EXT_WARPS) {
         const int strip = task % p.nstrips, chunk = task / p.nstrips;
-        // lane l holds columns xa = xs + 2l and xb = xa + 1; the warp owns
-        // xs + 1 .. xs + EXT_OWN (lane 0's a and lane 31's b are its halo)
-        const int xs = strip * EXT_OWN - 1;
-        const int xa = xs + EXT_V * lane, xb = xa + 1;
-        const int ca = min(max(xa, 0), nx - 1), cb = min(max(xb, 0), nx - 1);
-        const bool own_a = lane >= 1 && xa < nx;
-        const bool own_b = lane <= 30 && xb < nx;
-        const int y0 = chunk * EXT_H, y1 = min(y0 + EXT_H, ny);
-        const bool src_strip = !(xs + 1 + EXT_OWN <= p.bandx_lo || xs + 1 > p.bandx_hi);
-        // rows y0 - 1 (up) and y0 (centre), clamped at the field's edges
-        ExtCell ua, ub, a, b;
+        const int xs = strip * EXT_OWN - EXT_V;
+        s.xa = xs + EXT_V * lane;
+        s.xb = s.xa + 1;
+        s.ca = min(max(s.xa, 0), nx - 1);
+        s.cb = min(max(s.xb, 0), nx - 1);
+        s.cv = min(max(s.xa, 0), nx - 2);
+        s.own = lane >= 1 && lane <= 30 && s.xa < nx;
+        s.own_b = s.own && s.xb < nx;
+        const int y0 = chunk * p.H;
+        s.y1 = min(y0 + p.H, ny);
+        s.thr = s.own ? (s.tm < p.Tm ? s.tm : p.Tm) : INFINITY;
+        const bool src_strip = k.q_scale != 0.0 && xs + 32 * EXT_V > p.bandx_lo &&
+                               xs <= p.bandx_hi;
+        double Q[EXT_R][2];
         {
-            const size_t ru = (size_t)max(y0 - 1, 0) * nx, rc = (size_t)y0 * nx;
-            ua = ext_cell<KM>(__ldg(Tin + ru + ca), L, p.L, kmult);
-            ub = ext_cell<KM>(__ldg(Tin + ru + cb), L, p.L, kmult);
-            a = ext_cell<KM>(__ldg(Tin + rc + ca), L, p.L, kmult);
-            b = ext_cell<KM>(__ldg(Tin + rc + cb), L, p.L, kmult);
-        }
-        double Fua = ext_flux(ua, a), Fub = ext_flux(ub, b);
-        // the next EXT_PF rows in flight (a global load's latency spans
-        // several rows' arithmetic)
-        double Qa[EXT_PF], Qb[EXT_PF];
+            // rows y0 - 1 (up) and y0 (centre), clamped at the field's edges
+            double t0, t1, u0, u1;
+            ext_load<VEC>(Tin, nx, ny, y0 - 1, s, t0, t1);
+            ext_load<VEC>(Tin, nx, ny, y0, s, u0, u1);
 #pragma unroll
-        for (int i = 0; i < EXT_PF; ++i) {
-            const size_t r = (size_t)min(y0 + 1 + i, ny - 1) * nx;
-            Qa[i] = __ldg(Tin + r + ca);
-            Qb[i] = __ldg(Tin + r + cb);
+            for (int i = 0; i < EXT_R; ++i)
+                ext_load<VEC>(Tin, nx, ny, y0 + 1 + i, s, Q[i][0], Q[i][1]);
+            const ExtCell ua = ext_cell<KM>(t0, L, p.L, k.kmult);
+            const ExtCell ub = ext_cell<KM>(t1, L, p.L, k.kmult);
+            s.a = ext_cell<KM>(u0, L, p.L, k.kmult);
+            s.b = ext_cell<KM>(u1, L, p.L, k.kmult);
+            s.Fua = ext_flux(ua, s.a);
+            s.Fub = ext_flux(ub, s.b);
         }
-#pragma unroll EXT_PF
-        for (int y = y0; y < y1; ++y) {
-            const double Tda = Qa[0], Tdb = Qb[0];
-#pragma unroll
-            for (int i = 0; i < EXT_PF - 1; ++i) { Qa[i] = Qa[i + 1]; Qb[i] = Qb[i + 1]; }
-            // row y + EXT_PF + 1 is the lower neighbour of the task's row
-            // y + EXT_PF: needed while that row is < y1
-            if (y + EXT_PF < y1) {
-                const size_t r = (size_t)min(y + EXT_PF + 1, ny - 1) * nx;
-                Qa[EXT_PF - 1] = __ldg(Tin + r + ca);
-                Qb[EXT_PF - 1] = __ldg(Tin + r + cb);
-            }
-            const ExtCell da = ext_cell<KM>(Tda, L, p.L, kmult);
-            const ExtCell db = ext_cell<KM>(Tdb, L, p.L, kmult);
-            // x faces: a|b inside the lane, b|next lane's a, and the previous
-            // lane's b|a as this lane's left face; y faces: down, carried up
-            const double Fab = ext_flux(a, b);
-            const double TR = __shfl_down_sync(0xffffffffu, a.T, 1);
-            const double kR = __shfl_down_sync(0xffffffffu, a.k, 1);
-            const double FbR = __dmul_rn(__dadd_rn(b.k, kR), __dsub_rn(TR, b.T));
-            const double FLa = __shfl_up_sync(0xffffffffu, FbR, 1);
-            const double Fda = ext_flux(a, da), Fdb = ext_flux(b, db);
-            const double diva = fma(__dsub_rn(Fda, Fua), p.hy, __dmul_rn(__dsub_rn(Fab, FLa), p.hx));
-            const double divb = fma(__dsub_rn(Fdb, Fub), p.hy, __dmul_rn(__dsub_rn(FbR, Fab), p.hx));
-            double qa = 0.0, qb = 0.0;
-            if (src_strip && y >= p.band_lo && y <= p.band_hi && k.q_scale != 0.0) {
-                qa = ext_source(xa, y, k, p.r2_cut);
-                qb = ext_source(xb, y, k, p.r2_cut);
-            }
-            double va = ext_update(a, diva, qa, k, p, L);
-            double vb = ext_update(b, divb, qb, k, p, L);
-            if (p.bc == 1) {
-                const bool ey = y == 0 || y == ny - 1;
-                if (ey || xa == 0 || xa == nx - 1) va = p.T_edge;
-                if (ey || xb == 0 || xb == nx - 1) vb = p.T_edge;
-            }
-            double* row = Tout + (size_t)y * nx;
-            if (own_a) row[xa] = va;
-            if (own_b) row[xb] = vb;
-            if constexpr (REDUCE) {
-                // a lane meets its cells in increasing index order (rows
-                // down, a before b): strict '>' keeps the first maximum; NaN
-                // never wins
-                if (own_a && va > tm) { tm = va; ag = (long long)y * nx + xa; }
-                if (own_b && vb > tm) { tm = vb; ag = (long long)y * nx + xb; }
-                if (__any_sync(0xffffffffu, (own_a && va > p.Tm) || (own_b && vb > p.Tm)) &&
-                    lane == 0) {
-                    mn = min(mn, y);
-                    mx = max(mx, y);
-                }
-            }
-            // shift the rows
-            Fua = Fda; Fub = Fdb;
-            a = da; b = db;
+        s.cfa = s.cfb = 0.0;
+        if (src_strip && s.y1 > p.band_lo && y0 <= p.band_hi) {
+            s.cfa = ext_factor(s.xa, k.dx, k.x_l, k.inv_r0_sq, p.r2_cut);
+            s.cfb = ext_factor(s.xb, k.dx, k.x_l, k.inv_r0_sq, p.r2_cut);
+        }
+#pragma unroll 1
+        for (int y = y0; y < s.y1; y += EXT_R) {
+            if (src_strip && y + EXT_R > p.band_lo && y <= p.band_hi)
+                ext_block<REDUCE, KM, SAMET, VEC, true>(Tin, Tout, p, L, y, s, Q, lane);
+            else
+                ext_block<REDUCE, KM, SAMET, VEC, false>(Tin, Tout, p, L, y, s, Q, lane);
         }
     }
     if constexpr (REDUCE) {
-        mn = __shfl_sync(0xffffffffu, mn, 0);
-        mx = __shfl_sync(0xffffffffu, mx, 0);
+        double tm = s.tm;
+        long long ag = s.py < 0 ? N : (long long)s.py * nx + s.px;
+        int mn = s.mn, mx = s.mx;
         partial_warp_reduce(tm, ag, mn, mx);
         if (lane == 0) red[wid] = Partial{tm, ag, mn, mx};
         __syncthreads();
@@ -409,12 +507,27 @@ ext_step_kernel(const double* __restrict__ Tin, double* __restrict__ Tout,
     }
 }
 
+template <bool REDUCE, bool KM, bool SAMET>
+cudaError_t launch_ext_v(bool vec, int grid, const double* Tin, double* Tout, const ExtParams& p,
+                         cudaStream_t stream) {
+    constexpr int threads = EXT_WARPS * 32;
+    if (vec)
+        ext_step_kernel<REDUCE, KM, SAMET, true><<<grid, threads, 0, stream>>>(Tin, Tout, p);
+    else
+        ext_step_kernel<REDUCE, KM, SAMET, false><<<grid, threads, 0, stream>>>(Tin, Tout, p);
+    return cudaGetLastError();
+}
 template <bool REDUCE>
 cudaError_t launch_ext_t(bool km, int grid, const double* Tin, double* Tout, const ExtParams& p,
                          cudaStream_t stream) {
-    if (km) ext_step_kernel<REDUCE, true><<<grid, EXT_WARPS * 32, 0, stream>>>(Tin, Tout, p);
-    else ext_step_kernel<REDUCE, false><<<grid, EXT_WARPS * 32, 0, stream>>>(Tin, Tout, p);
-    return cudaGetLastError();
+    // even rows on 16-byte boundaries: 16-byte loads and stores
+    const bool vec = p.k.nx % 2 == 0 && reinterpret_cast<uintptr_t>(Tin) % 16 == 0 &&
+                     reinterpret_cast<uintptr_t>(Tout) % 16 == 0;
+    if (p.k.Tamb == p.k.Tsub)
+        return km ? launch_ext_v<REDUCE, true, true>(vec, grid, Tin, Tout, p, stream)
+                  : launch_ext_v<REDUCE, false, true>(vec, grid, Tin, Tout, p, stream);
+    return km ? launch_ext_v<REDUCE, true, false>(vec, grid, Tin, Tout, p, stream)
+              : launch_ext_v<REDUCE, false, false>(vec, grid, Tin, Tout, p, stream);
 }
 
 cudaError_t launch_ext_step(const double* Tin, double* Tout, const StepConst& k, int bc,
@@ -438,8 +551,21 @@ cudaError_t launch_ext_step(const double* Tin, double* Tout, const StepConst& k,
     p.r2_cut = c.r2_cut;
     laser_band(c, &las, 1, &p.band_lo, &p.band_hi, &p.bandx_lo, &p.bandx_hi);
     p.nstrips = (k.nx + EXT_OWN - 1) / EXT_OWN;
-    p.ntasks = p.nstrips * ((k.ny + EXT_H - 1) / EXT_H);
+    // 8..64 rows per task, in whole blocks, with the fewest waves x rows over
+    // the resident warps (two CTAs per SM), the taller on a tie
+    const long long warps = 2ll * EXT_WARPS * sm_count();
+    long long best = -1;
+    p.H = 8;
+    for (int h = 8; h <= EXT_H; h += EXT_R) {
+        const long long tasks = (long long)((k.ny + h - 1) / h) * p.nstrips;
+        const long long cost = ((tasks + warps - 1) / warps) * (h + 4);
+        if (best < 0 || cost <= best) { best = cost; p.H = h; }
+    }
+    p.ntasks = p.nstrips * ((k.ny + p.H - 1) / p.H);
     int grid = (p.ntasks + EXT_WARPS - 1) / EXT_WARPS;
+    // resident CTAs only: a warp goes on to its next task (in a later chunk, as
+    // its peak's tie rule needs) without leaving its place
+    if (p.nstrips <= warps) grid = std::min(grid, 2 * sm_count());
     const bool km = k.kmult > 1.0;
     const bool reduce = ring || ref_out;
     if (ref_out) {
