@@ -51,48 +51,10 @@ __device__ __forceinline__ void st_global_v4f_pred(float* p, const float* v, boo
                  :: "l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"((int)pred));
 }
 
-// ---- packed pairs of f32 -----------------------------------------------------
-// sm_100a executes two f32 operations per instruction on a 64-bit register
-// pair, each rounded as its scalar form.  These kernels are bound by
-// instruction issue, so the fast body holds and updates its four cells per
-// lane as two pairs; only what needs a neighbour across a pair's seam stays
-// scalar (the horizontal differences and sums, whose results land in pairs).
-typedef unsigned long long p2;
-__device__ __forceinline__ p2 p2_pack(float a, float b) {
-    p2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float p2_a(p2 v) {
-    float a, b;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-    return a;
-}
-__device__ __forceinline__ float p2_b(p2 v) {
-    float a, b;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-    return b;
-}
-__device__ __forceinline__ p2 p2_add(p2 a, p2 b) {
-    p2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ p2 p2_mul(p2 a, p2 b) {
-    p2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ p2 p2_fma(p2 a, p2 b, p2 c) {
-    p2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ p2 p2_sub(p2 a, p2 b) {
-    p2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
+// These kernels are bound by instruction issue, so the fast body holds and
+// updates its four cells per lane as two pairs; only what needs a neighbour
+// across a pair's seam stays scalar (the horizontal differences and sums,
+// whose results land in pairs).
 inline p2 p2_host(float v) {            // both halves v
     unsigned int b;
     std::memcpy(&b, &v, sizeof(b));

@@ -958,12 +958,32 @@ wgrad_row_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     if (warp == 1) tmem_free(tmem, 128);
 }
 
-// dW[co][tap * 32 + ci] and db[co] from the CTA records, summed in CTA order.
-__global__ void wgrad_row_reduce(const float* partial, int nrec, float* dw, float* db) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= WR_REC) return;
+// Sum of column e of `nrec` records of `stride` floats, by a block of 32
+// columns x 8 row groups (threadIdx.x, threadIdx.y): each group sums every
+// eighth record in order, then the groups are summed in order (the result
+// depends on nrec alone).  One thread per column walked a thousand records
+// alone: 44 us for a 1024-record sum of 1184 columns.
+__device__ __forceinline__ float sum_records(const float* partial, int nrec, int stride, int e,
+                                             bool in) {
+    __shared__ float part[8][33];
     float s = 0.0f;
-    for (int r = 0; r < nrec; ++r) s += partial[size_t(r) * WR_REC + e];
+    if (in) {
+#pragma unroll 8
+        for (int r = threadIdx.y; r < nrec; r += 8) s += partial[size_t(r) * stride + e];
+    }
+    part[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    s = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += part[i][threadIdx.x];
+    return s;
+}
+
+// dW[co][tap * 32 + ci] and db[co] from the CTA records.
+__global__ void wgrad_row_reduce(const float* partial, int nrec, float* dw, float* db) {
+    const int e = blockIdx.x * 32 + threadIdx.x;
+    const float s = sum_records(partial, nrec, WR_REC, e, e < WR_REC);
+    if (e >= WR_REC || threadIdx.y != 0) return;
     if (e < 9216) {
         const int co = e & 31, row = e >> 5, dy = row / 96, m = row % 96;
         dw[co * 288 + (dy * 3 + (m >> 5)) * 32 + (m & 31)] = s;
@@ -991,181 +1011,408 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* g, int B, int H, int W,
     ConvArgs a{};
     a.B = B; a.H = H; a.W = W; a.err = err;
     wgrad_row_kernel<<<grid, CT_THREADS, smem, s>>>(xm, gm, a, partial, (int)nu, xtiles, runs);
-    wgrad_row_reduce<<<(WR_REC + 255) / 256, 256, 0, s>>>(partial, grid, dw, db);
+    wgrad_row_reduce<<<(WR_REC + 31) / 32, dim3(32, 8), 0, s>>>(partial, grid, dw, db);
     return cudaGetLastError();
 }
 
-// ---- weight gradients of the 4 -> 32 and 32 -> 1 layers, CUDA cores ---------
+// ---- weight gradients of the 4 -> 32 and 32 -> 1 layers ----------------------
 //
-// Too narrow for 128-row tensor-core tiles (36 and 1 real rows): each thread
-// owns fixed sums over the pixels of its CTA's runs of rows, read from three
-// input rows and one gradient row staged in shared memory.
-//   32 -> 1 : 288 threads, one (tap, input channel) each; thread 0 also the
-//             bias.  Per pixel: one input value, one (broadcast) gradient.
-//   4 -> 32 : 148 of 160 threads, (tap, input channel) x 8 output channels,
-//             and 4 threads the bias of 8 channels each.
-// Each CTA writes its record in the gradient's own order (dW[co][tap][ci],
-// then db); a second kernel sums the records in CTA order.
-template <int CIN, int COUT>
-struct WgSmall {
-    static constexpr int NOUT = 9 * CIN * COUT + COUT;
-    static constexpr int THREADS = CIN == 32 ? 288 : 160;
-    static constexpr int RUN = 8;    // output rows per unit: enough CTAs to hide latency
-};
+// 36 and 1 real rows are too narrow for 128-row tcgen05 tiles; warp-level
+// bf16 MMAs (m16n8k16, fp32 accumulators) fit them, K running over 16 pixels.
+// Eight warps, one 16-pixel chunk of a 128-pixel row each; rows are loaded a
+// row ahead into registers and staged in shared memory, one barrier per row.
+//   4 -> 32 : M = 16 rows of one dy: two pixels' four channels are 16 bytes,
+//             so an 8 x 8 transposed matrix load at pixel p brings taps
+//             dx = 0, 1 and one at p + 2 tap dx = 2; its junk rows (dx = 3)
+//             are set to ones and give the bias.  N = 32 output channels.
+//             Matrix loads need 16-byte rows: odd pixels read a second copy of
+//             the row, shifted by one pixel.
+//   32 -> 1 : M = 32 input channels of an input row's pixels, N = the nine
+//             taps: the gradient of rows y - 1 .. y + 1 shifted by dx.
+// Each CTA writes one record in the gradient's own order (dW[co][tap][ci],
+// then db); a second kernel sums the records.  Bound by the 32-channel
+// operand's bytes; on CUDA cores (one fp32 product per thread and pixel) the
+// two took 417 and 152 us at 32 x 256^2.
+constexpr int WS_THREADS = 256;
+constexpr int WS_WARPS = WS_THREADS / 32;
+constexpr int WS_RUN = 8;              // rows per unit
+constexpr int WS_PITCH = 80;           // bytes per pixel of a staged 32-channel row (conflict-free)
+constexpr int WS_XROW = 1088;          // bytes of a staged 4-channel row copy (132 pixels)
+constexpr int WS_COPY = WS_XROW + 64;  // the shifted copy, 64 bytes off in the banks
 
-template <int CIN, int COUT>
-__global__ void __launch_bounds__((WgSmall<CIN, COUT>::THREADS))
-wgrad_small_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, int W,
-                   int nunits, int xtiles, int runs, float* partial) {
-    static_assert((CIN == 32 && COUT == 1) || (CIN == 4 && COUT == 32), "narrow layers");
-    constexpr int NOUT = WgSmall<CIN, COUT>::NOUT;
-    // input rows as bf16 (pixel p of a slot is column xt * 128 - 1 + p), the
-    // gradient row as fp32
-    __shared__ __align__(16) uint16_t sx[3][CR_PX][CIN];
-    __shared__ __align__(16) float sg[128][COUT];
-    const int t = threadIdx.x;
-    // outputs of this thread
-    int tap = 0, ci = 0, cb = 0;
-    bool bias = false, active = true;
-    if constexpr (CIN == 32) {
-        tap = t >> 5;
-        ci = t & 31;
-        bias = t == 0;
-    } else {
-        const int tc = t >> 2;
-        cb = (t & 3) * 8;
-        active = tc <= 36;
-        bias = tc == 36;
-        tap = bias ? 0 : tc >> 2;
-        ci = tc & 3;
-    }
-    const int dy = tap / 3, dx = tap % 3;
-    float acc[COUT == 32 ? 8 : 1];
-    float bacc = 0.0f;
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
+                                         uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
+                 "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// A unit: 128-pixel column tile xt of image b, rows [y0, y0 + n).
+struct WsUnit { int x0, b, y0, n; };
+__device__ __forceinline__ WsUnit ws_unit(int u, int xtiles, int runs, int H) {
+    WsUnit r;
+    r.x0 = (u % xtiles) * 128;
+    r.b = (u / xtiles) / runs;
+    r.y0 = ((u / xtiles) % runs) * WS_RUN;
+    r.n = min(WS_RUN, H - r.y0);
+    return r;
+}
+// A 32-channel row's 128 pixels, two 16-byte units per thread (zero off the image).
+__device__ __forceinline__ void ws_load32(uint4 (&v)[2], const bf16* src, int b, int y, int x0,
+                                          int H, int W, int t) {
 #pragma unroll
-    for (int c = 0; c < (COUT == 32 ? 8 : 1); ++c) acc[c] = 0.0f;
+    for (int i = 0; i < 2; ++i) {
+        const int u = t + i * WS_THREADS, px = x0 + (u >> 2);
+        v[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (y >= 0 && y < H && px < W)
+            v[i] = __ldg(reinterpret_cast<const uint4*>(
+                src + ((size_t(b) * H + y) * W + px) * 32 + (u & 3) * 8));
+    }
+}
+__device__ __forceinline__ void ws_store32(unsigned char* row, const uint4 (&v)[2], int t) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int u = t + i * WS_THREADS;
+        *reinterpret_cast<uint4*>(row + (u >> 2) * WS_PITCH + (u & 3) * 16) = v[i];
+    }
+}
 
-    auto stage_x = [&](int slot, int b, int y, int x0) {
-        // 16-byte units of CIN channels: CIN = 32: 4 per pixel; CIN = 4: half
-        // a unit per pixel, so 8-byte units
-        if constexpr (CIN == 32) {
-            for (int i = t; i < CR_PX * 4; i += blockDim.x) {
-                const int p = i >> 2, q = i & 3, xx = x0 - 1 + p;
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (y >= 0 && y < H && xx >= 0 && xx < W)
-                    v = __ldg(reinterpret_cast<const uint4*>(
-                        x + ((size_t(b) * H + y) * W + xx) * 32 + q * 8));
-                *reinterpret_cast<uint4*>(&sx[slot][p][q * 8]) = v;
-            }
-        } else {
-            for (int p = t; p < CR_PX; p += blockDim.x) {
-                const int xx = x0 - 1 + p;
-                uint2 v = make_uint2(0u, 0u);
-                if (y >= 0 && y < H && xx >= 0 && xx < W)
-                    v = __ldg(reinterpret_cast<const uint2*>(x + ((size_t(b) * H + y) * W + xx) * 4));
-                *reinterpret_cast<uint2*>(&sx[slot][p][0]) = v;
-            }
+// Records of the two layers, in floats.
+constexpr int WS_IN_REC = 32 * 36 + 32, WS_OUT_REC = 9 * 32 + 1;
+
+__global__ void __launch_bounds__(WS_THREADS, 2)
+wgrad_in_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, int W, int nunits,
+                int xtiles, int runs, float* partial) {
+    __shared__ __align__(128) unsigned char sx[4][WS_COPY + WS_XROW];  // input rows (ring), two copies
+    __shared__ __align__(128) unsigned char sg[2][128 * WS_PITCH];
+    __shared__ float sum[WS_IN_REC];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    float acc[3][4][4];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[d][n][i] = 0.0f;
+
+    // input row y: pixel q of the slot is column x0 - 1 + q
+    auto load_x = [&](const WsUnit& r, int y) {
+        uint2 v = make_uint2(0u, 0u);
+        const int xx = r.x0 - 1 + t;
+        if (t < 132 && y >= 0 && y < H && xx >= 0 && xx < W)
+            v = __ldg(reinterpret_cast<const uint2*>(x + ((size_t(r.b) * H + y) * W + xx) * 4));
+        return v;
+    };
+    auto store_x = [&](int slot, uint2 v) {
+        if (t < 132) {
+            *reinterpret_cast<uint2*>(&sx[slot][8 * t]) = v;
+            if (t > 0) *reinterpret_cast<uint2*>(&sx[slot][WS_COPY + 8 * (t - 1)]) = v;
         }
     };
-    auto stage_g = [&](int b, int y, int x0) {
-        for (int i = t; i < 128 * COUT; i += blockDim.x) {
-            const int p = i / COUT, c = i % COUT, xx = x0 + p;
-            float v = 0.0f;
-            if (xx < W) {
-                const uint16_t u = reinterpret_cast<const uint16_t*>(g)[((size_t(b) * H + y) * W + xx) * COUT + c];
-                v = __uint_as_float(uint32_t(u) << 16);
-            }
-            sg[p][c] = v;
-        }
-    };
+    // this lane's row of the transposed loads: pixel k of the chunk
+    const int k = 16 * warp + (lane & 7) + ((lane >> 4) & 1) * 8;
+    const uint32_t xoff = (k & 1 ? WS_COPY + 8 * (k - 1) : 8 * k) + ((lane >> 3) & 1) * 16;
+    const uint32_t goff = (16 * warp + (lane & 15)) * WS_PITCH + (lane >> 4) * 16;
 
-    constexpr int RUN = WgSmall<CIN, COUT>::RUN;
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-        RowUnit r;
-        r.xt = u % xtiles;
-        r.b = (u / xtiles) / runs;
-        r.y0 = ((u / xtiles) % runs) * RUN;
-        r.n = min(RUN, H - r.y0);
-        const int x0 = r.xt * 128;
-        stage_x(0, r.b, r.y0 - 1, x0);
-        stage_x(1, r.b, r.y0, x0);
+        const WsUnit r = ws_unit(u, xtiles, runs, H);
+        uint4 gv[2];
+        ws_load32(gv, g, r.b, r.y0, r.x0, H, W, t);
+        const uint2 xa = load_x(r, r.y0 - 1), xb = load_x(r, r.y0);
+        uint2 xv = load_x(r, r.y0 + 1);
+        __syncthreads();                       // the previous unit's rows are read
+        store_x(0, xa);
+        store_x(1, xb);
         for (int j = 0; j < r.n; ++j) {
-            stage_x((j + 2) % 3, r.b, r.y0 + j + 1, x0);
-            stage_g(r.b, r.y0 + j, x0);
+            // row j: input rows in slots j, j + 1, j + 2 (mod 4)
+            store_x((j + 2) & 3, xv);
+            ws_store32(sg[j & 1], gv, t);
             __syncthreads();
-            if (active) {
-                const uint16_t* xr = &sx[(j + dy) % 3][dx][ci];
-                if constexpr (COUT == 1) {
-#pragma unroll 8
-                    for (int p = 0; p < 128; ++p) {
-                        const float gv = sg[p][0];
-                        acc[0] = fmaf(__uint_as_float(uint32_t(xr[p * CIN]) << 16), gv, acc[0]);
-                        if (bias) bacc += gv;
-                    }
-                } else {
-#pragma unroll 4
-                    for (int p = 0; p < 128; ++p) {
-                        const float4 g0 = *reinterpret_cast<const float4*>(&sg[p][cb]);
-                        const float4 g1 = *reinterpret_cast<const float4*>(&sg[p][cb + 4]);
-                        const float xv = bias ? 1.0f : __uint_as_float(uint32_t(xr[p * CIN]) << 16);
-                        acc[0] = fmaf(xv, g0.x, acc[0]); acc[1] = fmaf(xv, g0.y, acc[1]);
-                        acc[2] = fmaf(xv, g0.z, acc[2]); acc[3] = fmaf(xv, g0.w, acc[3]);
-                        acc[4] = fmaf(xv, g1.x, acc[4]); acc[5] = fmaf(xv, g1.y, acc[5]);
-                        acc[6] = fmaf(xv, g1.z, acc[6]); acc[7] = fmaf(xv, g1.w, acc[7]);
-                    }
-                }
+            if (j + 1 < r.n) {
+                ws_load32(gv, g, r.b, r.y0 + j + 1, r.x0, H, W, t);
+                xv = load_x(r, r.y0 + j + 2);
             }
-            __syncthreads();
-        }
-    }
-    float* rec = partial + size_t(blockIdx.x) * NOUT;
-    if constexpr (COUT == 1) {
-        rec[tap * 32 + ci] = acc[0];
-        if (bias) rec[288] = bacc;
-    } else if (active) {
+            uint32_t b0[4], b1[4];             // channels 0-15, 16-31
+            const uint32_t ga = smem_u32(sg[j & 1]) + goff;
+            ldsm4t(b0, ga);
+            ldsm4t(b1, ga + 32);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            if (bias) rec[9 * 4 * 32 + cb + c] = acc[c];
-            else      rec[(cb + c) * 36 + tap * 4 + ci] = acc[c];
+            for (int d = 0; d < 3; ++d) {
+                uint32_t a[4];
+                ldsm4t(a, smem_u32(sx[(j + d) & 3]) + xoff);
+                if (lane >= 16) a[1] = a[3] = 0x3f803f80u;      // rows 12-15: ones (bf16)
+                mma16816(acc[d][0], a, b0[0], b0[1]);
+                mma16816(acc[d][1], a, b0[2], b0[3]);
+                mma16816(acc[d][2], a, b1[0], b1[1]);
+                mma16816(acc[d][3], a, b1[2], b1[3]);
+            }
         }
     }
+    // the CTA's record: the warps' sums in warp order
+    for (int i = t; i < WS_IN_REC; i += WS_THREADS) sum[i] = 0.0f;
+    for (int w = 0; w < WS_WARPS; ++w) {
+        __syncthreads();
+        if (w != warp) continue;
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int m = (lane >> 2) + (i >> 1) * 8;
+                    const int co = n * 8 + (lane & 3) * 2 + (i & 1);
+                    if (m < 12) sum[co * 36 + (d * 3 + (m >> 2)) * 4 + (m & 3)] += acc[d][n][i];
+                    else if (m == 12 && d == 1) sum[32 * 36 + co] += acc[d][n][i];
+                }
+    }
+    __syncthreads();
+    for (int i = t; i < WS_IN_REC; i += WS_THREADS)
+        partial[size_t(blockIdx.x) * WS_IN_REC + i] = sum[i];
+}
+
+__global__ void __launch_bounds__(WS_THREADS, 2)
+wgrad_out_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, int W, int nunits,
+                 int xtiles, int runs, float* partial) {
+    __shared__ __align__(128) unsigned char sx[2][128 * WS_PITCH];
+    // gradient rows (ring): value i is column x0 - 2 + i; the second copy
+    // holds value i + 1 at i, for pairs that start at an odd index
+    __shared__ __align__(16) uint16_t sg[4][2][136];
+    __shared__ float sum[WS_OUT_REC + 31];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    float acc[2][2][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.0f;
+    float bias = 0.0f;
+
+    auto load_g = [&](const WsUnit& r, int y) {
+        uint16_t v = 0;
+        const int xx = r.x0 - 2 + t;
+        if (t < 132 && y >= 0 && y < H && xx >= 0 && xx < W)
+            v = __ldg(reinterpret_cast<const uint16_t*>(g) + (size_t(r.b) * H + y) * W + xx);
+        return v;
+    };
+    auto store_g = [&](int slot, uint16_t v) {
+        if (t < 132) {
+            sg[slot][0][t] = v;
+            if (t > 0) sg[slot][1][t - 1] = v;
+        }
+    };
+    // columns of the two 8-wide tap tiles: n < 6 of the first are (dy, dx) =
+    // (n / 3, n % 3), n < 3 of the second (2, n); tap (dy, dx) of input pixel
+    // k meets gradient row y - dy + 1, column k - dx + 1 (value k - dx + 3)
+    const int n = lane >> 2, dx0 = n % 3, dy0 = n / 3;
+    const uint32_t xoff = (16 * warp + (lane & 7) + ((lane >> 4) & 1) * 8) * WS_PITCH +
+                          ((lane >> 3) & 1) * 16;
+    auto pair = [&](const uint16_t (*row)[136], int i) {
+        return *reinterpret_cast<const uint32_t*>(&row[i & 1][i & ~1]);
+    };
+
+    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+        const WsUnit r = ws_unit(u, xtiles, runs, H);
+        uint4 xv[2];
+        ws_load32(xv, x, r.b, r.y0, r.x0, H, W, t);
+        const uint16_t ga = load_g(r, r.y0 - 1), gb = load_g(r, r.y0);
+        uint16_t gv = load_g(r, r.y0 + 1);
+        __syncthreads();
+        store_g(0, ga);
+        store_g(1, gb);
+        // the bias: each gradient value once, by the tile and row that own it
+        const bool mine = t >= 2 && t < 130;
+        if (mine) bias += __uint_as_float(uint32_t(gb) << 16);
+        for (int j = 0; j < r.n; ++j) {
+            // input row j: gradient rows j - 1, j, j + 1 in slots j, j + 1, j + 2 (mod 4)
+            store_g((j + 2) & 3, gv);
+            if (mine && j + 1 < r.n) bias += __uint_as_float(uint32_t(gv) << 16);
+            ws_store32(sx[j & 1], xv, t);
+            __syncthreads();
+            if (j + 1 < r.n) {
+                ws_load32(xv, x, r.b, r.y0 + j + 1, r.x0, H, W, t);
+                gv = load_g(r, r.y0 + j + 2);
+            }
+            const int k0 = 16 * warp + (lane & 3) * 2;
+            uint32_t b[2][2] = {{0u, 0u}, {0u, 0u}};
+            if (n < 6) {
+                const auto* row = sg[(j + 2 - dy0) & 3];
+                b[0][0] = pair(row, k0 - dx0 + 3);
+                b[0][1] = pair(row, k0 + 8 - dx0 + 3);
+            }
+            if (n < 3) {
+                const auto* row = sg[j & 3];
+                b[1][0] = pair(row, k0 - n + 3);
+                b[1][1] = pair(row, k0 + 8 - n + 3);
+            }
+            const uint32_t xa = smem_u32(sx[j & 1]) + xoff;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                uint32_t a[4];
+                ldsm4t(a, xa + 32 * m);
+                mma16816(acc[m][0], a, b[0][0], b[0][1]);
+                mma16816(acc[m][1], a, b[1][0], b[1][1]);
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bias += __shfl_xor_sync(0xffffffffu, bias, o);
+    for (int i = t; i < WS_OUT_REC; i += WS_THREADS) sum[i] = 0.0f;
+    for (int w = 0; w < WS_WARPS; ++w) {
+        __syncthreads();
+        if (w != warp) continue;
+        if (lane == 0) sum[288] += bias;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int ci = m * 16 + (lane >> 2) + (i >> 1) * 8;
+                    const int c = (lane & 3) * 2 + (i & 1);
+                    if (c < (q == 0 ? 6 : 3)) sum[(q * 6 + c) * 32 + ci] += acc[m][q][i];
+                }
+    }
+    __syncthreads();
+    for (int i = t; i < WS_OUT_REC; i += WS_THREADS)
+        partial[size_t(blockIdx.x) * WS_OUT_REC + i] = sum[i];
 }
 
 template <int NOUT, int NW>
 __global__ void wgrad_small_reduce(const float* partial, int nrec, float* dw, float* db) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= NOUT) return;
-    float s = 0.0f;
-    for (int r = 0; r < nrec; ++r) s += partial[size_t(r) * NOUT + e];
+    const int e = blockIdx.x * 32 + threadIdx.x;
+    const float s = sum_records(partial, nrec, NOUT, e, e < NOUT);
+    if (e >= NOUT || threadIdx.y != 0) return;
     if (e < NW) dw[e] = s;
     else        db[e - NW] = s;
 }
 
-template <int CIN, int COUT>
-cudaError_t launch_wgrad_small(const bf16* x, const bf16* g, int B, int H, int W, float* dw,
-                               float* db, float* partial, cudaStream_t s) {
-    constexpr int NOUT = WgSmall<CIN, COUT>::NOUT;
-    if (reinterpret_cast<uintptr_t>(x) % 16 != 0) return cudaErrorNotSupported;
-    constexpr int RUN = WgSmall<CIN, COUT>::RUN;
+template <int NOUT, int NW, typename KERN>
+cudaError_t launch_wgrad_small(KERN kern, const bf16* x, const bf16* g, int B, int H, int W,
+                               float* dw, float* db, float* partial, cudaStream_t s) {
+    if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(g) % 16 != 0)
+        return cudaErrorNotSupported;
     const int xtiles = (W + 127) / 128;
-    const int runs = (H + RUN - 1) / RUN;
+    const int runs = (H + WS_RUN - 1) / WS_RUN;
     const long long nu = (long long)xtiles * runs * B;
-    const long long P = (long long)B * H * W;
     if (nu >= (1ll << 31)) return cudaErrorInvalidValue;
-    const int grid = (int)std::min<long long>({nu, 8ll * sm_count(), (long long)WR_MAX_CTAS, P});
-    wgrad_small_kernel<CIN, COUT><<<grid, WgSmall<CIN, COUT>::THREADS, 0, s>>>(
-        x, g, H, W, (int)nu, xtiles, runs, partial);
-    wgrad_small_reduce<NOUT, 9 * CIN * COUT><<<(NOUT + 255) / 256, 256, 0, s>>>(partial, grid, dw, db);
+    const int grid = (int)std::min<long long>(nu, 2ll * sm_count());
+    kern<<<grid, WS_THREADS, 0, s>>>(x, g, H, W, (int)nu, xtiles, runs, partial);
+    wgrad_small_reduce<NOUT, NW><<<(NOUT + 31) / 32, dim3(32, 8), 0, s>>>(partial, grid, dw, db);
+    return cudaGetLastError();
+}
+
+// ---- input gradient of the 32 -> 1 layer --------------------------------------
+//
+// One input channel: nine products per output are too few for a tensor-core
+// tile (K = 9 of 64, gathered by threads: 237 us at 32 x 256^2).  A thread owns
+// eight channels of a pixel with their 72 weights in registers, as pairs; a
+// block walks rows of a 64-pixel tile with the three gradient rows in shared
+// memory.  Bound by the pre-activation and output bytes (128 B per pixel).
+constexpr int DX_PX = 64, DX_RUN = 16;
+
+__global__ void __launch_bounds__(256, 2)
+dx_out_kernel(const bf16* __restrict__ g, const bf16* __restrict__ w,
+              const bf16* __restrict__ pre, bf16* __restrict__ out, int H, int W, int nunits,
+              int xtiles, int runs) {
+    __shared__ float sg[4][DX_PX + 2];
+    const int t = threadIdx.x, px = t >> 2, c0 = (t & 3) * 8;
+    // dx weights [ci][64]: k = tap
+    p2 wt[9][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+            wt[k][q] = p2_pack(float(w[(c0 + 2 * q) * 64 + k]), float(w[(c0 + 2 * q + 1) * 64 + k]));
+    const p2 CA = p2_pack(GELU_CA, GELU_CA), C1 = p2_pack(GELU_C, GELU_C),
+             CA3 = p2_pack(3.0f * GELU_CA, 3.0f * GELU_CA), H2 = p2_pack(0.5f, 0.5f),
+             ONE = p2_pack(1.0f, 1.0f);
+    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+        const int x0 = (u % xtiles) * DX_PX, b = (u / xtiles) / runs;
+        const int y0 = ((u / xtiles) % runs) * DX_RUN, n = min(DX_RUN, H - y0);
+        auto load = [&](int y) {
+            const int xx = x0 - 1 + t;
+            uint16_t v = 0;
+            if (t < DX_PX + 2 && y >= 0 && y < H && xx >= 0 && xx < W)
+                v = __ldg(reinterpret_cast<const uint16_t*>(g) + (size_t(b) * H + y) * W + xx);
+            return __uint_as_float(uint32_t(v) << 16);
+        };
+        const float g0 = load(y0 - 1), g1 = load(y0);
+        float gv = load(y0 + 1);
+        __syncthreads();                       // the previous unit's rows are read
+        if (t < DX_PX + 2) {
+            sg[0][t] = g0;
+            sg[1][t] = g1;
+        }
+        const int xx = x0 + px;
+        const size_t p0 = ((size_t(b) * H + y0) * W + xx) * 32 + c0;
+        uint4 pv = make_uint4(0u, 0u, 0u, 0u);
+        if (xx < W) pv = __ldg(reinterpret_cast<const uint4*>(pre + p0));
+        for (int j = 0; j < n; ++j) {
+            if (t < DX_PX + 2) sg[(j + 2) & 3][t] = gv;
+            __syncthreads();
+            const uint4 cur = pv;
+            if (j + 1 < n) {
+                gv = load(y0 + j + 2);
+                if (xx < W) pv = __ldg(reinterpret_cast<const uint4*>(pre + p0 + size_t(j + 1) * W * 32));
+            }
+            p2 acc[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const float v = sg[(j + k / 3) & 3][px + k % 3];
+                const p2 vv = p2_pack(v, v);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[q] = p2_fma(vv, wt[k][q], acc[q]);
+            }
+            // times gelu'(pre) (gelu_grad's operations, two at a time)
+            const uint32_t in[4] = {cur.x, cur.y, cur.z, cur.w};
+            uint32_t o[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const p2 v = p2_pack(__uint_as_float(in[q] << 16),
+                                     __uint_as_float(in[q] & 0xffff0000u));
+                const p2 v2 = p2_mul(v, v);
+                const p2 a = p2_mul(v, p2_fma(v2, CA, C1));
+                const p2 th = p2_pack(tanh_approx(p2_a(a)), tanh_approx(p2_b(a)));
+                const p2 du = p2_fma(v2, CA3, C1);
+                const p2 om = p2_sub(ONE, p2_mul(th, th));
+                const p2 d = p2_fma(p2_mul(p2_mul(H2, v), om), du, p2_fma(H2, th, H2));
+                const p2 r = p2_mul(acc[q], d);
+                o[q] = pack_bf16(p2_a(r), p2_b(r));
+            }
+            if (xx < W)
+                *reinterpret_cast<uint4*>(out + p0 + size_t(j) * W * 32) =
+                    make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+}
+
+cudaError_t launch_dx_out(const ConvArgs& a, cudaStream_t s) {
+    if (reinterpret_cast<uintptr_t>(a.pre_in) % 16 != 0 ||
+        reinterpret_cast<uintptr_t>(a.out) % 16 != 0)
+        return cudaErrorNotSupported;
+    const int xtiles = (a.W + DX_PX - 1) / DX_PX, runs = (a.H + DX_RUN - 1) / DX_RUN;
+    const long long nu = (long long)xtiles * runs * a.B;
+    if (nu >= (1ll << 31)) return cudaErrorNotSupported;
+    const int grid = (int)std::min<long long>(nu, 2ll * sm_count());
+    dx_out_kernel<<<grid, 256, 0, s>>>(static_cast<const bf16*>(a.x), a.w, a.pre_in,
+                                       static_cast<bf16*>(a.out), a.H, a.W, (int)nu, xtiles, runs);
     return cudaGetLastError();
 }
 
 cudaError_t launch_wgrad_in(const bf16* x, const bf16* g, int B, int H, int W, float* dw, float* db,
                             float* partial, cudaStream_t s) {
-    return launch_wgrad_small<4, 32>(x, g, B, H, W, dw, db, partial, s);
+    return launch_wgrad_small<WS_IN_REC, 32 * 36>(wgrad_in_kernel, x, g, B, H, W, dw, db, partial,
+                                                  s);
 }
 cudaError_t launch_wgrad_out(const bf16* x, const bf16* g, int B, int H, int W, float* dw,
                              float* db, float* partial, cudaStream_t s) {
-    return launch_wgrad_small<32, 1>(x, g, B, H, W, dw, db, partial, s);
+    return launch_wgrad_small<WS_OUT_REC, 288>(wgrad_out_kernel, x, g, B, H, W, dw, db, partial, s);
 }
 
 template <int N, int EPI>
@@ -1277,7 +1524,9 @@ int lpbf_b200_sg_conv(int kind, const lpbf_b200_sg_conv_args* p, cudaStream_t st
             e = launch_conv32<16, EPI_LINEAR>(a, stream); break;
         case LPBF_SG_DX_OUT:
             if (!a.pre_in) return LPBF_ERR_ARG;
-            e = launch_conv<1, 32, EPI_DGELU>(a, stream); break;
+            e = g_conv_form == 0 ? launch_dx_out(a, stream) : cudaErrorNotSupported;
+            if (e == cudaErrorNotSupported) e = launch_conv<1, 32, EPI_DGELU>(a, stream);
+            break;
         case LPBF_SG_DX_HIDDEN:
             if (!a.pre_in) return LPBF_ERR_ARG;
             e = launch_conv32<32, EPI_DGELU>(a, stream); break;
