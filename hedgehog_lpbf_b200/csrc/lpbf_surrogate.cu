@@ -43,6 +43,7 @@ struct ConvArgs {
     void* out;              // GELU/DGELU: bf16 [P][N]; LINEAR: fp32 [P]
     int B, H, W;
     unsigned int* err;
+    int wide;               // activations on 32-byte boundaries: 256-bit accesses
 };
 
 template <int CIN> struct KOf { static constexpr int K = CIN == 32 ? 288 : 64;
@@ -310,33 +311,47 @@ __device__ __forceinline__ void epilogue16(const ConvArgs& a, size_t p, int c0, 
         static_cast<float*>(a.out)[p] = v[0] + (a.bias ? a.bias[0] : 0.0f);
     } else {
         uint32_t o[8], pr[8];
+        // 256-bit accesses where the buffers allow: a lane's 32 bytes are one
+        // sector, and two 16-byte stores would write it in halves
         if constexpr (EPI == EPI_GELU) {
 #pragma unroll
             for (int c = 0; c < 16; c += 2) {
-                const float v0 = v[c] + bias[c], v1 = v[c + 1] + bias[c + 1];
-                pr[c / 2] = pack_bf16(v0, v1);
-                o[c / 2] = pack_bf16(gelu(v0), gelu(v1));
+                const p2 x = p2_add(p2_pack(v[c], v[c + 1]), p2_pack(bias[c], bias[c + 1]));
+                const p2 y = gelu2(x);
+                pr[c / 2] = pack_bf16(p2_a(x), p2_b(x));
+                o[c / 2] = pack_bf16(p2_a(y), p2_b(y));
             }
         } else {
-            const uint4* src = reinterpret_cast<const uint4*>(a.pre_in + p * N + c0);
-            const uint4 u0 = __ldg(src), u1 = __ldg(src + 1);
-            const uint32_t w[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+            const bf16* src = a.pre_in + p * N + c0;
+            uint32_t w[8];
+            if (a.wide) {
+                ld_global_nc_32b(w, src);
+            } else {
+                const uint4 u0 = __ldg(reinterpret_cast<const uint4*>(src));
+                const uint4 u1 = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+                w[0] = u0.x; w[1] = u0.y; w[2] = u0.z; w[3] = u0.w;
+                w[4] = u1.x; w[5] = u1.y; w[6] = u1.z; w[7] = u1.w;
+            }
 #pragma unroll
             for (int c = 0; c < 16; c += 2) {
-                const float g0 = __uint_as_float(w[c / 2] << 16);
-                const float g1 = __uint_as_float(w[c / 2] & 0xffff0000u);
-                o[c / 2] = pack_bf16(v[c] * gelu_grad(g0), v[c + 1] * gelu_grad(g1));
+                const p2 g = p2_pack(__uint_as_float(w[c / 2] << 16),
+                                     __uint_as_float(w[c / 2] & 0xffff0000u));
+                const p2 y = p2_mul(p2_pack(v[c], v[c + 1]), gelu_grad2(g));
+                o[c / 2] = pack_bf16(p2_a(y), p2_b(y));
             }
         }
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + p * N + c0);
-        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-        if constexpr (EPI == EPI_GELU) {
-            if (a.pre_out) {
-                uint4* dp = reinterpret_cast<uint4*>(a.pre_out + p * N + c0);
-                dp[0] = make_uint4(pr[0], pr[1], pr[2], pr[3]);
-                dp[1] = make_uint4(pr[4], pr[5], pr[6], pr[7]);
+        auto store = [&](bf16* base, const uint32_t (&q)[8]) {
+            bf16* dst = base + p * N + c0;
+            if (a.wide) {
+                st_global_32b(dst, q);
+            } else {
+                reinterpret_cast<uint4*>(dst)[0] = make_uint4(q[0], q[1], q[2], q[3]);
+                reinterpret_cast<uint4*>(dst)[1] = make_uint4(q[4], q[5], q[6], q[7]);
             }
+        };
+        store(static_cast<bf16*>(a.out), o);
+        if constexpr (EPI == EPI_GELU) {
+            if (a.pre_out) store(a.pre_out, pr);
         }
     }
 }
@@ -1329,9 +1344,6 @@ dx_out_kernel(const bf16* __restrict__ g, const bf16* __restrict__ w,
 #pragma unroll
         for (int k = 0; k < 9; ++k)
             wt[k][q] = p2_pack(float(w[(c0 + 2 * q) * 64 + k]), float(w[(c0 + 2 * q + 1) * 64 + k]));
-    const p2 CA = p2_pack(GELU_CA, GELU_CA), C1 = p2_pack(GELU_C, GELU_C),
-             CA3 = p2_pack(3.0f * GELU_CA, 3.0f * GELU_CA), H2 = p2_pack(0.5f, 0.5f),
-             ONE = p2_pack(1.0f, 1.0f);
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const int x0 = (u % xtiles) * DX_PX, b = (u / xtiles) / runs;
         const int y0 = ((u / xtiles) % runs) * DX_RUN, n = min(DX_RUN, H - y0);
@@ -1369,20 +1381,14 @@ dx_out_kernel(const bf16* __restrict__ g, const bf16* __restrict__ w,
 #pragma unroll
                 for (int q = 0; q < 4; ++q) acc[q] = p2_fma(vv, wt[k][q], acc[q]);
             }
-            // times gelu'(pre) (gelu_grad's operations, two at a time)
+            // times gelu'(pre)
             const uint32_t in[4] = {cur.x, cur.y, cur.z, cur.w};
             uint32_t o[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const p2 v = p2_pack(__uint_as_float(in[q] << 16),
                                      __uint_as_float(in[q] & 0xffff0000u));
-                const p2 v2 = p2_mul(v, v);
-                const p2 a = p2_mul(v, p2_fma(v2, CA, C1));
-                const p2 th = p2_pack(tanh_approx(p2_a(a)), tanh_approx(p2_b(a)));
-                const p2 du = p2_fma(v2, CA3, C1);
-                const p2 om = p2_sub(ONE, p2_mul(th, th));
-                const p2 d = p2_fma(p2_mul(p2_mul(H2, v), om), du, p2_fma(H2, th, H2));
-                const p2 r = p2_mul(acc[q], d);
+                const p2 r = p2_mul(acc[q], gelu_grad2(v));
                 o[q] = pack_bf16(p2_a(r), p2_b(r));
             }
             if (xx < W)
@@ -1505,6 +1511,8 @@ int lpbf_b200_sg_conv(int kind, const lpbf_b200_sg_conv_args* p, cudaStream_t st
     a.H = p->height;
     a.W = p->width;
     a.err = p->err;
+    a.wide = (reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.pre_in) |
+              reinterpret_cast<uintptr_t>(a.pre_out)) % 32 == 0;
     cudaError_t e;
     switch (kind) {
         case LPBF_SG_FWD_IN:

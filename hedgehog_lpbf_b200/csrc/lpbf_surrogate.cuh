@@ -157,6 +157,38 @@ __device__ __forceinline__ float gelu_grad(float x) {
     return fmaf(hx * fmaf(-t, t, 1.0f), du, fmaf(0.5f, t, 0.5f));
 }
 
+// The same, two values at a time (packed f32: half the issue slots; the same
+// operations, so the same bits).
+__device__ __forceinline__ p2 p2_tanh(p2 v) {
+    return p2_pack(tanh_approx(p2_a(v)), tanh_approx(p2_b(v)));
+}
+__device__ __forceinline__ p2 gelu2(p2 x) {
+    const p2 u = p2_mul(x, p2_fma(p2_mul(x, x), p2_pack(GELU_CA, GELU_CA), p2_pack(GELU_C, GELU_C)));
+    const p2 hx = p2_mul(p2_pack(0.5f, 0.5f), x);
+    return p2_fma(hx, p2_tanh(u), hx);
+}
+__device__ __forceinline__ p2 gelu_grad2(p2 x) {
+    const p2 half = p2_pack(0.5f, 0.5f), one = p2_pack(1.0f, 1.0f), c = p2_pack(GELU_C, GELU_C);
+    const p2 x2 = p2_mul(x, x);
+    const p2 t = p2_tanh(p2_mul(x, p2_fma(x2, p2_pack(GELU_CA, GELU_CA), c)));
+    const p2 du = p2_fma(x2, p2_pack(3.0f * GELU_CA, 3.0f * GELU_CA), c);
+    const p2 om = p2_fma(t ^ 0x8000000080000000ull, t, one);
+    return p2_fma(p2_mul(p2_mul(half, x), om), du, p2_fma(half, t, half));
+}
+// 32 bytes (a full sector) per lane.
+__device__ __forceinline__ void st_global_32b(void* p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :: "l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]),
+                    "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void ld_global_nc_32b(uint32_t (&v)[8], const void* p) {
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
+                   "=r"(v[6]), "=r"(v[7])
+                 : "l"(p));
+}
+
 // Opt kernel KERN in to `bytes` of dynamic shared memory on the current
 // device, once per device (the attribute belongs to each device's context).
 template <auto KERN>
