@@ -304,9 +304,26 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // Epilogue of 16 accumulator columns (channels c0 .. c0 + 15) of pixel p.
 // GELU: bias, pre-activation and activation out (bf16); LINEAR: channel 0
 // plus bias (fp32); DGELU: times gelu'(pre_in) (bf16).
+// DGELU: the pre-activations of epilogue16's 16 channels (loaded ahead of the
+// accumulator's wait where there is one).
+template <int N, int EPI>
+__device__ __forceinline__ void load_pre16(const ConvArgs& a, size_t p, int c0, uint32_t (&w)[8]) {
+    if constexpr (EPI == EPI_DGELU) {
+        const bf16* src = a.pre_in + p * N + c0;
+        if (a.wide) {
+            ld_global_nc_32b(w, src);
+        } else {
+            const uint4 u0 = __ldg(reinterpret_cast<const uint4*>(src));
+            const uint4 u1 = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+            w[0] = u0.x; w[1] = u0.y; w[2] = u0.z; w[3] = u0.w;
+            w[4] = u1.x; w[5] = u1.y; w[6] = u1.z; w[7] = u1.w;
+        }
+    }
+}
+
 template <int N, int EPI>
 __device__ __forceinline__ void epilogue16(const ConvArgs& a, size_t p, int c0, const float* v,
-                                           const float* bias) {
+                                           const float* bias, const uint32_t (&w)[8]) {
     if constexpr (EPI == EPI_LINEAR) {
         static_cast<float*>(a.out)[p] = v[0] + (a.bias ? a.bias[0] : 0.0f);
     } else {
@@ -322,16 +339,6 @@ __device__ __forceinline__ void epilogue16(const ConvArgs& a, size_t p, int c0, 
                 o[c / 2] = pack_bf16(p2_a(y), p2_b(y));
             }
         } else {
-            const bf16* src = a.pre_in + p * N + c0;
-            uint32_t w[8];
-            if (a.wide) {
-                ld_global_nc_32b(w, src);
-            } else {
-                const uint4 u0 = __ldg(reinterpret_cast<const uint4*>(src));
-                const uint4 u1 = __ldg(reinterpret_cast<const uint4*>(src) + 1);
-                w[0] = u0.x; w[1] = u0.y; w[2] = u0.z; w[3] = u0.w;
-                w[4] = u1.x; w[5] = u1.y; w[6] = u1.z; w[7] = u1.w;
-            }
 #pragma unroll
             for (int c = 0; c < 16; c += 2) {
                 const p2 g = p2_pack(__uint_as_float(w[c / 2] << 16),
@@ -443,7 +450,9 @@ conv_tma_kernel(const __grid_constant__ CUtensorMap xmap, const ConvArgs a, int 
             const int y = row % a.H, b = row / a.H;
             const int x = xt * 128 + q * 32 + lane;
             if (!active || x >= a.W) continue;
-            epilogue16<N, EPI>(a, (size_t(b) * a.H + y) * a.W + x, 16 * h, v, bias);
+            uint32_t w[8];
+            load_pre16<N, EPI>(a, (size_t(b) * a.H + y) * a.W + x, 16 * h, w);
+            epilogue16<N, EPI>(a, (size_t(b) * a.H + y) * a.W + x, 16 * h, v, bias, w);
         }
     }
     if (!ok && a.err) atomicOr(a.err, 1u);
@@ -740,6 +749,10 @@ conv_row_kernel(const __grid_constant__ CUtensorMap xmap, const ConvArgs a, int 
             const RowUnit r = row_unit(u, xtiles, runs, a.H);
             for (int j = 0; j < r.n; ++j, ++o) {
                 const int acc = o % CR_NACC;
+                const int x = r.xt * 128 + q * 32 + lane;
+                const size_t p = (size_t(r.b) * a.H + r.y0 + j) * a.W + x;
+                uint32_t w[8];
+                if (active && x < a.W) load_pre16<N, EPI>(a, p, 16 * h, w);
                 if (!__all_sync(0xffffffffu,
                                 mbar_wait_bounded(&tfull[acc], (o / CR_NACC) & 1))) {
                     ok = false;
@@ -752,9 +765,8 @@ conv_row_kernel(const __grid_constant__ CUtensorMap xmap, const ConvArgs a, int 
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&tempty[acc]);
-                const int x = r.xt * 128 + q * 32 + lane;
                 if (!active || x >= a.W) continue;
-                epilogue16<N, EPI>(a, (size_t(r.b) * a.H + r.y0 + j) * a.W + x, 16 * h, v, bias);
+                epilogue16<N, EPI>(a, p, 16 * h, v, bias, w);
             }
         }
     }
@@ -1034,8 +1046,9 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* g, int B, int H, int W,
 //
 // 36 and 1 real rows are too narrow for 128-row tcgen05 tiles; warp-level
 // bf16 MMAs (m16n8k16, fp32 accumulators) fit them, K running over 16 pixels.
-// Eight warps, one 16-pixel chunk of a 128-pixel row each; rows are loaded a
-// row ahead into registers and staged in shared memory, one barrier per row.
+// Eight warps, one 16-pixel chunk of a 128-pixel row each; rows are copied
+// asynchronously into shared memory WS_AHEAD rows ahead (one row ahead kept
+// 16 KB per SM in flight: 2.1 TB/s), one barrier per row.
 //   4 -> 32 : M = 16 rows of one dy: two pixels' four channels are 16 bytes,
 //             so an 8 x 8 transposed matrix load at pixel p brings taps
 //             dx = 0, 1 and one at p + 2 tap dx = 2; its junk rows (dx = 3)
@@ -1051,6 +1064,7 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* g, int B, int H, int W,
 constexpr int WS_THREADS = 256;
 constexpr int WS_WARPS = WS_THREADS / 32;
 constexpr int WS_RUN = 8;              // rows per unit
+constexpr int WS_AHEAD = 3, WS_ROWS = 4;     // rows copied ahead; slots of the 32-channel row ring
 constexpr int WS_PITCH = 80;           // bytes per pixel of a staged 32-channel row (conflict-free)
 constexpr int WS_XROW = 1088;          // bytes of a staged 4-channel row copy (132 pixels)
 constexpr int WS_COPY = WS_XROW + 64;  // the shifted copy, 64 bytes off in the banks
@@ -1077,23 +1091,32 @@ __device__ __forceinline__ WsUnit ws_unit(int u, int xtiles, int runs, int H) {
     r.n = min(WS_RUN, H - r.y0);
     return r;
 }
-// A 32-channel row's 128 pixels, two 16-byte units per thread (zero off the image).
-__device__ __forceinline__ void ws_load32(uint4 (&v)[2], const bf16* src, int b, int y, int x0,
+// Asynchronous copies into shared memory (zeros where !in), and their groups.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 :: "r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;"
+                 :: "r"(smem_u32(dst)), "l"(src), "r"(in ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory");
+}
+// A 32-channel row's 128 pixels into a padded slot, two 16-byte units per
+// thread (zero off the image).
+__device__ __forceinline__ void ws_copy32(unsigned char* row, const bf16* src, int b, int y, int x0,
                                           int H, int W, int t) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int u = t + i * WS_THREADS, px = x0 + (u >> 2);
-        v[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (y >= 0 && y < H && px < W)
-            v[i] = __ldg(reinterpret_cast<const uint4*>(
-                src + ((size_t(b) * H + y) * W + px) * 32 + (u & 3) * 8));
-    }
-}
-__device__ __forceinline__ void ws_store32(unsigned char* row, const uint4 (&v)[2], int t) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int u = t + i * WS_THREADS;
-        *reinterpret_cast<uint4*>(row + (u >> 2) * WS_PITCH + (u & 3) * 16) = v[i];
+        const bool in = y >= 0 && y < H && px < W;
+        cp_async16(row + (u >> 2) * WS_PITCH + (u & 3) * 16,
+                   in ? src + ((size_t(b) * H + y) * W + px) * 32 + (u & 3) * 8 : src, in);
     }
 }
 
@@ -1103,9 +1126,11 @@ constexpr int WS_IN_REC = 32 * 36 + 32, WS_OUT_REC = 9 * 32 + 1;
 __global__ void __launch_bounds__(WS_THREADS, 2)
 wgrad_in_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, int W, int nunits,
                 int xtiles, int runs, float* partial) {
-    __shared__ __align__(128) unsigned char sx[4][WS_COPY + WS_XROW];  // input rows (ring), two copies
-    __shared__ __align__(128) unsigned char sg[2][128 * WS_PITCH];
-    __shared__ float sum[WS_IN_REC];
+    extern __shared__ __align__(128) unsigned char ws_smem[];
+    auto sg = reinterpret_cast<unsigned char (*)[128 * WS_PITCH]>(ws_smem);       // [WS_ROWS]
+    auto sx = reinterpret_cast<unsigned char (*)[WS_COPY + WS_XROW]>(
+        ws_smem + WS_ROWS * 128 * WS_PITCH);          // input rows (ring of 8), two copies
+    float* const sum = reinterpret_cast<float*>(ws_smem);                 // after the last row
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     float acc[3][4][4];
 #pragma unroll
@@ -1115,18 +1140,14 @@ wgrad_in_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, i
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[d][n][i] = 0.0f;
 
-    // input row y: pixel q of the slot is column x0 - 1 + q
-    auto load_x = [&](const WsUnit& r, int y) {
-        uint2 v = make_uint2(0u, 0u);
-        const int xx = r.x0 - 1 + t;
-        if (t < 132 && y >= 0 && y < H && xx >= 0 && xx < W)
-            v = __ldg(reinterpret_cast<const uint2*>(x + ((size_t(r.b) * H + y) * W + xx) * 4));
-        return v;
-    };
-    auto store_x = [&](int slot, uint2 v) {
+    // input row y into a slot: pixel q of the slot is column x0 - 1 + q
+    auto copy_x = [&](const WsUnit& r, int y, int slot) {
         if (t < 132) {
-            *reinterpret_cast<uint2*>(&sx[slot][8 * t]) = v;
-            if (t > 0) *reinterpret_cast<uint2*>(&sx[slot][WS_COPY + 8 * (t - 1)]) = v;
+            const int xx = r.x0 - 1 + t;
+            const bool in = y >= 0 && y < H && xx >= 0 && xx < W;
+            const bf16* src = in ? x + ((size_t(r.b) * H + y) * W + xx) * 4 : x;
+            cp_async8(&sx[slot][8 * t], src, in);
+            if (t > 0) cp_async8(&sx[slot][WS_COPY + 8 * (t - 1)], src, in);
         }
     };
     // this lane's row of the transposed loads: pixel k of the chunk
@@ -1136,30 +1157,32 @@ wgrad_in_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, i
 
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const WsUnit r = ws_unit(u, xtiles, runs, H);
-        uint4 gv[2];
-        ws_load32(gv, g, r.b, r.y0, r.x0, H, W, t);
-        const uint2 xa = load_x(r, r.y0 - 1), xb = load_x(r, r.y0);
-        uint2 xv = load_x(r, r.y0 + 1);
         __syncthreads();                       // the previous unit's rows are read
-        store_x(0, xa);
-        store_x(1, xb);
-        for (int j = 0; j < r.n; ++j) {
-            // row j: input rows in slots j, j + 1, j + 2 (mod 4)
-            store_x((j + 2) & 3, xv);
-            ws_store32(sg[j & 1], gv, t);
-            __syncthreads();
-            if (j + 1 < r.n) {
-                ws_load32(gv, g, r.b, r.y0 + j + 1, r.x0, H, W, t);
-                xv = load_x(r, r.y0 + j + 2);
+        copy_x(r, r.y0 - 1, 0);
+        copy_x(r, r.y0, 1);
+        // group i: gradient row i and the input row below it (slot i + 2 mod 8)
+        auto copy_row = [&](int i) {
+            if (i < r.n) {
+                copy_x(r, r.y0 + i + 1, (i + 2) & 7);
+                ws_copy32(sg[i % WS_ROWS], g, r.b, r.y0 + i, r.x0, H, W, t);
             }
+            cp_commit();
+        };
+#pragma unroll
+        for (int i = 0; i < WS_AHEAD; ++i) copy_row(i);
+        for (int j = 0; j < r.n; ++j) {
+            // row j: input rows in slots j, j + 1, j + 2 (mod 8)
+            cp_wait<WS_AHEAD - 1>();
+            __syncthreads();
+            copy_row(j + WS_AHEAD);            // its slots were read before the barrier
             uint32_t b0[4], b1[4];             // channels 0-15, 16-31
-            const uint32_t ga = smem_u32(sg[j & 1]) + goff;
+            const uint32_t ga = smem_u32(sg[j % WS_ROWS]) + goff;
             ldsm4t(b0, ga);
             ldsm4t(b1, ga + 32);
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 uint32_t a[4];
-                ldsm4t(a, smem_u32(sx[(j + d) & 3]) + xoff);
+                ldsm4t(a, smem_u32(sx[(j + d) & 7]) + xoff);
                 if (lane >= 16) a[1] = a[3] = 0x3f803f80u;      // rows 12-15: ones (bf16)
                 mma16816(acc[d][0], a, b0[0], b0[1]);
                 mma16816(acc[d][1], a, b0[2], b0[3]);
@@ -1169,6 +1192,8 @@ wgrad_in_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, i
         }
     }
     // the CTA's record: the warps' sums in warp order
+    cp_wait<0>();
+    __syncthreads();
     for (int i = t; i < WS_IN_REC; i += WS_THREADS) sum[i] = 0.0f;
     for (int w = 0; w < WS_WARPS; ++w) {
         __syncthreads();
@@ -1193,10 +1218,11 @@ wgrad_in_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, i
 __global__ void __launch_bounds__(WS_THREADS, 2)
 wgrad_out_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, int W, int nunits,
                  int xtiles, int runs, float* partial) {
-    __shared__ __align__(128) unsigned char sx[2][128 * WS_PITCH];
+    extern __shared__ __align__(128) unsigned char ws_smem[];
+    auto sx = reinterpret_cast<unsigned char (*)[128 * WS_PITCH]>(ws_smem);       // [WS_ROWS]
     // gradient rows (ring): value i is column x0 - 2 + i; the second copy
     // holds value i + 1 at i, for pairs that start at an odd index
-    __shared__ __align__(16) uint16_t sg[4][2][136];
+    __shared__ __align__(16) uint16_t sg[8][2][136];
     __shared__ float sum[WS_OUT_REC + 31];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     float acc[2][2][4];
@@ -1233,39 +1259,47 @@ wgrad_out_kernel(const bf16* __restrict__ x, const bf16* __restrict__ g, int H, 
 
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const WsUnit r = ws_unit(u, xtiles, runs, H);
-        uint4 xv[2];
-        ws_load32(xv, x, r.b, r.y0, r.x0, H, W, t);
-        const uint16_t ga = load_g(r, r.y0 - 1), gb = load_g(r, r.y0);
-        uint16_t gv = load_g(r, r.y0 + 1);
-        __syncthreads();
-        store_g(0, ga);
-        store_g(1, gb);
+        __syncthreads();                       // the previous unit's rows are read
+        auto copy_row = [&](int i) {
+            if (i < r.n) ws_copy32(sx[i % WS_ROWS], x, r.b, r.y0 + i, r.x0, H, W, t);
+            cp_commit();
+        };
+#pragma unroll
+        for (int i = 0; i < WS_AHEAD; ++i) copy_row(i);
+        // gradient rows through registers (2-byte values): row y0 - 1 + i in
+        // slot i mod 8, rows up to j + 1 stored and three more in flight
+        const uint16_t g0 = load_g(r, r.y0 - 1), g1 = load_g(r, r.y0);
+        uint16_t gq[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) gq[i] = load_g(r, r.y0 + 1 + i);
+        store_g(0, g0);
+        store_g(1, g1);
         // the bias: each gradient value once, by the tile and row that own it
         const bool mine = t >= 2 && t < 130;
-        if (mine) bias += __uint_as_float(uint32_t(gb) << 16);
+        if (mine) bias += __uint_as_float(uint32_t(g1) << 16);
         for (int j = 0; j < r.n; ++j) {
-            // input row j: gradient rows j - 1, j, j + 1 in slots j, j + 1, j + 2 (mod 4)
-            store_g((j + 2) & 3, gv);
-            if (mine && j + 1 < r.n) bias += __uint_as_float(uint32_t(gv) << 16);
-            ws_store32(sx[j & 1], xv, t);
+            // input row j: gradient rows j - 1, j, j + 1 in slots j, j + 1, j + 2 (mod 8)
+            store_g((j + 2) & 7, gq[0]);
+            if (mine && j + 1 < r.n) bias += __uint_as_float(uint32_t(gq[0]) << 16);
+            gq[0] = gq[1];
+            gq[1] = gq[2];
+            gq[2] = load_g(r, r.y0 + j + 4);
+            cp_wait<WS_AHEAD - 1>();
             __syncthreads();
-            if (j + 1 < r.n) {
-                ws_load32(xv, x, r.b, r.y0 + j + 1, r.x0, H, W, t);
-                gv = load_g(r, r.y0 + j + 2);
-            }
+            copy_row(j + WS_AHEAD);
             const int k0 = 16 * warp + (lane & 3) * 2;
             uint32_t b[2][2] = {{0u, 0u}, {0u, 0u}};
             if (n < 6) {
-                const auto* row = sg[(j + 2 - dy0) & 3];
+                const auto* row = sg[(j + 2 - dy0) & 7];
                 b[0][0] = pair(row, k0 - dx0 + 3);
                 b[0][1] = pair(row, k0 + 8 - dx0 + 3);
             }
             if (n < 3) {
-                const auto* row = sg[j & 3];
+                const auto* row = sg[j & 7];
                 b[1][0] = pair(row, k0 - n + 3);
                 b[1][1] = pair(row, k0 + 8 - n + 3);
             }
-            const uint32_t xa = smem_u32(sx[j & 1]) + xoff;
+            const uint32_t xa = smem_u32(sx[j % WS_ROWS]) + xoff;
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 uint32_t a[4];
@@ -1307,8 +1341,8 @@ __global__ void wgrad_small_reduce(const float* partial, int nrec, float* dw, fl
     else        db[e - NW] = s;
 }
 
-template <int NOUT, int NW, typename KERN>
-cudaError_t launch_wgrad_small(KERN kern, const bf16* x, const bf16* g, int B, int H, int W,
+template <int NOUT, int NW, auto KERN>
+cudaError_t launch_wgrad_small(const bf16* x, const bf16* g, int B, int H, int W,
                                float* dw, float* db, float* partial, cudaStream_t s) {
     if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(g) % 16 != 0)
         return cudaErrorNotSupported;
@@ -1317,7 +1351,9 @@ cudaError_t launch_wgrad_small(KERN kern, const bf16* x, const bf16* g, int B, i
     const long long nu = (long long)xtiles * runs * B;
     if (nu >= (1ll << 31)) return cudaErrorInvalidValue;
     const int grid = (int)std::min<long long>(nu, 2ll * sm_count());
-    kern<<<grid, WS_THREADS, 0, s>>>(x, g, H, W, (int)nu, xtiles, runs, partial);
+    constexpr size_t smem = WS_ROWS * 128 * WS_PITCH + 8 * (WS_COPY + WS_XROW);
+    if (const cudaError_t e = smem_opt_in<KERN>(smem); e != cudaSuccess) return e;
+    KERN<<<grid, WS_THREADS, smem, s>>>(x, g, H, W, (int)nu, xtiles, runs, partial);
     wgrad_small_reduce<NOUT, NW><<<(NOUT + 31) / 32, dim3(32, 8), 0, s>>>(partial, grid, dw, db);
     return cudaGetLastError();
 }
@@ -1330,12 +1366,14 @@ cudaError_t launch_wgrad_small(KERN kern, const bf16* x, const bf16* g, int B, i
 // block walks rows of a 64-pixel tile with the three gradient rows in shared
 // memory.  Bound by the pre-activation and output bytes (128 B per pixel).
 constexpr int DX_PX = 64, DX_RUN = 16;
+constexpr int DX_AHEAD = 7;        // rows of pre-activations in flight per thread (own slots)
 
 __global__ void __launch_bounds__(256, 2)
 dx_out_kernel(const bf16* __restrict__ g, const bf16* __restrict__ w,
               const bf16* __restrict__ pre, bf16* __restrict__ out, int H, int W, int nunits,
               int xtiles, int runs) {
-    __shared__ float sg[4][DX_PX + 2];
+    __shared__ float sg[8][DX_PX + 2];
+    __shared__ __align__(16) uint4 spre[DX_AHEAD + 1][256];
     const int t = threadIdx.x, px = t >> 2, c0 = (t & 3) * 8;
     // dx weights [ci][64]: k = tap
     p2 wt[9][4];
@@ -1354,29 +1392,37 @@ dx_out_kernel(const bf16* __restrict__ g, const bf16* __restrict__ w,
                 v = __ldg(reinterpret_cast<const uint16_t*>(g) + (size_t(b) * H + y) * W + xx);
             return __uint_as_float(uint32_t(v) << 16);
         };
+        const int xx = x0 + px;
+        const size_t p0 = ((size_t(b) * H + y0) * W + xx) * 32 + c0;
+        auto copy_pre = [&](int i) {
+            const bool in = i < n && xx < W;
+            cp_async16(&spre[i % (DX_AHEAD + 1)][t], in ? pre + p0 + size_t(i) * W * 32 : pre, in);
+            cp_commit();
+        };
+#pragma unroll
+        for (int i = 0; i < DX_AHEAD; ++i) copy_pre(i);
         const float g0 = load(y0 - 1), g1 = load(y0);
-        float gv = load(y0 + 1);
+        float gq[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) gq[i] = load(y0 + 1 + i);
         __syncthreads();                       // the previous unit's rows are read
         if (t < DX_PX + 2) {
             sg[0][t] = g0;
             sg[1][t] = g1;
         }
-        const int xx = x0 + px;
-        const size_t p0 = ((size_t(b) * H + y0) * W + xx) * 32 + c0;
-        uint4 pv = make_uint4(0u, 0u, 0u, 0u);
-        if (xx < W) pv = __ldg(reinterpret_cast<const uint4*>(pre + p0));
         for (int j = 0; j < n; ++j) {
-            if (t < DX_PX + 2) sg[(j + 2) & 3][t] = gv;
+            if (t < DX_PX + 2) sg[(j + 2) & 7][t] = gq[0];
+            gq[0] = gq[1];
+            gq[1] = gq[2];
+            gq[2] = load(y0 + j + 4);
             __syncthreads();
-            const uint4 cur = pv;
-            if (j + 1 < n) {
-                gv = load(y0 + j + 2);
-                if (xx < W) pv = __ldg(reinterpret_cast<const uint4*>(pre + p0 + size_t(j + 1) * W * 32));
-            }
+            cp_wait<DX_AHEAD - 1>();           // a thread reads only its own copies
+            const uint4 cur = spre[j % (DX_AHEAD + 1)][t];
+            copy_pre(j + DX_AHEAD);
             p2 acc[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
             for (int k = 0; k < 9; ++k) {
-                const float v = sg[(j + k / 3) & 3][px + k % 3];
+                const float v = sg[(j + k / 3) & 7][px + k % 3];
                 const p2 vv = p2_pack(v, v);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) acc[q] = p2_fma(vv, wt[k][q], acc[q]);
@@ -1413,12 +1459,11 @@ cudaError_t launch_dx_out(const ConvArgs& a, cudaStream_t s) {
 
 cudaError_t launch_wgrad_in(const bf16* x, const bf16* g, int B, int H, int W, float* dw, float* db,
                             float* partial, cudaStream_t s) {
-    return launch_wgrad_small<WS_IN_REC, 32 * 36>(wgrad_in_kernel, x, g, B, H, W, dw, db, partial,
-                                                  s);
+    return launch_wgrad_small<WS_IN_REC, 32 * 36, wgrad_in_kernel>(x, g, B, H, W, dw, db, partial, s);
 }
 cudaError_t launch_wgrad_out(const bf16* x, const bf16* g, int B, int H, int W, float* dw,
                              float* db, float* partial, cudaStream_t s) {
-    return launch_wgrad_small<WS_OUT_REC, 288>(wgrad_out_kernel, x, g, B, H, W, dw, db, partial, s);
+    return launch_wgrad_small<WS_OUT_REC, 288, wgrad_out_kernel>(x, g, B, H, W, dw, db, partial, s);
 }
 
 template <int N, int EPI>

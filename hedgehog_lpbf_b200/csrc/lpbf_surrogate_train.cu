@@ -360,28 +360,58 @@ struct FeatArgs {
     double dx, dy, Tamb, m2r, r2_cut;
     SgLaser las[LPBF_SG_STEPS];
     double xm, ym;                   // laser position at the middle step
+    int bx0, bx1, by0, by1;          // cells any step's source can reach
+    int out8;                        // out on an 8-byte boundary
     bf16* out;                       // [ny][nx][4]
 };
 
-__global__ void features_kernel(const FeatArgs a) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= (long long)a.nx * a.ny) return;
-    const int x = (int)(i % a.nx), y = (int)(i / a.nx);
-    const double px = x * a.dx, py = y * a.dy;
-    double S = 0.0;
-#pragma unroll 4
-    for (int s = 0; s < LPBF_SG_STEPS; ++s) {
-        if (a.las[s].cs == 0.0) continue;
-        const double ddx = px - a.las[s].x, ddy = py - a.las[s].y;
-        const double r2 = ddx * ddx + ddy * ddy;
-        if (r2 < a.r2_cut) S += a.las[s].cs * exp(a.m2r * r2);
-    }
-    const float f0 = (float)((a.T[i] - a.Tamb) * (1.0 / LPBF_SG_T_SCALE));
-    const float f1 = (float)(S * (1.0 / LPBF_SG_S_SCALE));
-    const float f2 = fminf(fmaxf((float)((px - a.xm) * (1.0 / LPBF_SG_POS_SCALE)), -8.f), 8.f);
+// One row per block row, two pixels per thread.  Only the box [bx0, bx1] x
+// [by0, by1] (cells any step's source can reach) sums the 16 Gaussians: the
+// range test of every step at every cell took 46 us at 2048^2, for 67 MB that
+// take 10.
+constexpr int FEAT_PX = 2;
+__global__ void __launch_bounds__(256) features_kernel(const FeatArgs a) {
+    const int y = blockIdx.y + 65535 * blockIdx.z;
+    const int x0 = (blockIdx.x * 256 + threadIdx.x) * FEAT_PX;
+    if (y >= a.ny || x0 >= a.nx) return;
+    const double py = y * a.dy;
     const float f3 = fminf(fmaxf((float)((py - a.ym) * (1.0 / LPBF_SG_POS_SCALE)), -8.f), 8.f);
-    bf16* o = a.out + size_t(i) * 4;
-    o[0] = bf16(f0); o[1] = bf16(f1); o[2] = bf16(f2); o[3] = bf16(f3);
+    const size_t i0 = size_t(y) * a.nx + x0;
+    uint2 o[FEAT_PX];
+#pragma unroll
+    for (int v = 0; v < FEAT_PX; ++v) {
+        const int x = x0 + v;
+        const double px = x * a.dx;
+        double S = 0.0;
+        if (y >= a.by0 && y <= a.by1 && x >= a.bx0 && x <= a.bx1) {
+#pragma unroll 4
+            for (int s = 0; s < LPBF_SG_STEPS; ++s) {
+                if (a.las[s].cs == 0.0) continue;
+                const double ddx = px - a.las[s].x, ddy = py - a.las[s].y;
+                const double r2 = ddx * ddx + ddy * ddy;
+                if (r2 < a.r2_cut) S += a.las[s].cs * exp(a.m2r * r2);
+            }
+        }
+        const double T = x < a.nx ? __ldg(a.T + i0 + v) : a.Tamb;
+        const bf16 f0 = bf16((float)((T - a.Tamb) * (1.0 / LPBF_SG_T_SCALE)));
+        const bf16 f1 = bf16((float)(S * (1.0 / LPBF_SG_S_SCALE)));
+        const bf16 f2 = bf16(fminf(fmaxf((float)((px - a.xm) * (1.0 / LPBF_SG_POS_SCALE)), -8.f), 8.f));
+        const bf16 f4 = bf16(f3);
+        o[v] = make_uint2(uint32_t(f0.raw()) | uint32_t(f1.raw()) << 16,
+                          uint32_t(f2.raw()) | uint32_t(f4.raw()) << 16);
+    }
+    bf16* dst = a.out + i0 * 4;
+#pragma unroll
+    for (int v = 0; v < FEAT_PX; ++v)
+        if (x0 + v < a.nx) {
+            if (a.out8) {
+                *reinterpret_cast<uint2*>(dst + 4 * v) = o[v];
+            } else {
+                uint16_t* h = reinterpret_cast<uint16_t*>(dst + 4 * v);
+                h[0] = uint16_t(o[v].x); h[1] = uint16_t(o[v].x >> 16);
+                h[2] = uint16_t(o[v].y); h[3] = uint16_t(o[v].y >> 16);
+            }
+        }
 }
 
 // T += y * DT_SCALE (the super-step), or the target of a pair of snapshots.
@@ -592,15 +622,20 @@ int lpbf_b200_sg_features(const double* T, const StepConst* k, const lpbf_tick* 
     const Coef c = make_coef(*k, 0, k->Tamb, 0.0);
     a.m2r = c.m2r;
     a.r2_cut = c.r2_cut;
+    LaserSub las[LPBF_SG_STEPS];
     for (int s = 0; s < LPBF_SG_STEPS; ++s) {
         const LaserSub l = make_laser(*k, plan[s].x_l, plan[s].y_l, plan[s].q_scale);
         a.las[s] = SgLaser{l.x_l, l.y_l, l.cs};
+        las[s] = l;
     }
+    laser_band(c, las, LPBF_SG_STEPS, &a.by0, &a.by1, &a.bx0, &a.bx1);
+    a.out8 = reinterpret_cast<uintptr_t>(x4) % 8 == 0;
     a.xm = plan[LPBF_SG_STEPS / 2].x_l;
     a.ym = plan[LPBF_SG_STEPS / 2].y_l;
     a.out = static_cast<bf16*>(x4);
-    const long long n = (long long)k->nx * k->ny;
-    features_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(a);
+    const dim3 grid((unsigned)((k->nx + 256 * FEAT_PX - 1) / (256 * FEAT_PX)),
+                    (unsigned)std::min(k->ny, 65535), (unsigned)((k->ny + 65534) / 65535));
+    features_kernel<<<grid, 256, 0, stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? LPBF_OK : LPBF_ERR_CUDA;
 }
 
