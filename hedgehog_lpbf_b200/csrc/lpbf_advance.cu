@@ -241,8 +241,7 @@ cudaError_t launch_t(const double* Tin, double* Tout, const Coef& c, const Laser
     std::memset(&map, 0, sizeof(map));
     if (TMA && !tensor_map_f64(Tin, c.nx, c.ny, ADV_COLS, ADV_R, &map))
         return cudaErrorNotSupported;
-    kern<<<grid, ADV_WARPS * 32, smem, stream>>>(map, p);
-    return cudaGetLastError();
+    return launch_chained(kern, grid, ADV_WARPS * 32, smem, stream, map, p);
 }
 
 template <int K, bool SQ>

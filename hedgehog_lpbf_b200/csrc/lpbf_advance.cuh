@@ -942,6 +942,8 @@ advance_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ 
 
     WarpStrip<K, TMA, REDUCE, false, SQ ? 1 : 0> ws(p, &map, stages, bars, lane,
                                                     &s_red[REDUCE ? wid : 0]);
+    pdl_trigger();
+    pdl_wait();
     if (p.tasks) {
         // dynamic: lane 0 draws the next task for the warp
         for (;;) {

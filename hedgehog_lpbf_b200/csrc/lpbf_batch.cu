@@ -149,6 +149,8 @@ batch_kernel(const __grid_constant__ BatchLaunch L) {
     volatile TaskCtx* ctx = &s_ctx[wid];
     int bound = -1;                // scenario whose parameters sit in `par`
 
+    pdl_trigger();
+    pdl_wait();
     for (;;) {
         unsigned int tq = 0;
         if (lane == 0) tq = atomicAdd(&L.hdr->queue, 1u);
@@ -278,9 +280,8 @@ struct BatchKernelInfo {
         int grid = std::min(sm_count() * per_sm, (L.ntasks + ADV_WARPS - 1) / ADV_WARPS);
         grid = std::max(grid, 1);
         const size_t smem = STAGED ? ADV_SMEM_BYTES : 0;
-        if (L.sq_all) batch_kernel<K, ST, 1><<<grid, ADV_WARPS * 32, smem, s>>>(L);
-        else          batch_kernel<K, ST, 2><<<grid, ADV_WARPS * 32, smem, s>>>(L);
-        return cudaGetLastError();
+        return launch_chained(L.sq_all ? batch_kernel<K, ST, 1> : batch_kernel<K, ST, 2>, grid,
+                              ADV_WARPS * 32, smem, s, L);
     }
 };
 

@@ -103,21 +103,32 @@ constexpr int FIN_THREADS = 512;
 __global__ void finalize_cluster_kernel(const Partial* __restrict__ parts, int nblocks, int nx, int ny,
                         Partial* __restrict__ out);
 
-// Launch finalize_cluster_kernel as one cluster of FIN_CTAS CTAs.
+__global__ void finalize_small_kernel(const Partial* __restrict__ parts, int nblocks, int nx,
+                                      int ny, Partial* __restrict__ out);
+
+// Launch finalize_cluster_kernel as one cluster of FIN_CTAS CTAs, or, for up
+// to FIN_THREADS Partials (the unfused reduce's 256), one CTA: a cluster's
+// launch and two cluster barriers cost more than the reduction (4.9 us for
+// 256 Partials).
 inline cudaError_t launch_finalize(const Partial* parts, int nblocks, int nx, int ny,
                                    Partial* out, cudaStream_t stream) {
+    if (nblocks <= FIN_THREADS)
+        return launch_chained(finalize_small_kernel, 1, nblocks <= 256 ? 256 : FIN_THREADS, 0,
+                              stream, parts, nblocks, nx, ny, out);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(FIN_CTAS, 1, 1);
     cfg.blockDim = dim3(FIN_THREADS, 1, 1);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = FIN_CTAS;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, finalize_cluster_kernel, parts, nblocks, nx, ny, out);
 }
 
@@ -407,6 +418,8 @@ ext_step_kernel(const double* __restrict__ Tin, double* __restrict__ Tout,
         reinterpret_cast<double*>(&L)[threadIdx.x] =
             reinterpret_cast<const double*>(&p.L)[threadIdx.x];
     __syncthreads();
+    pdl_trigger();
+    pdl_wait();
     const int nx = k.nx, ny = k.ny;
     const long long N = (long long)nx * ny;
     ExtStrip s;
@@ -511,11 +524,9 @@ template <bool REDUCE, bool KM, bool SAMET>
 cudaError_t launch_ext_v(bool vec, int grid, const double* Tin, double* Tout, const ExtParams& p,
                          cudaStream_t stream) {
     constexpr int threads = EXT_WARPS * 32;
-    if (vec)
-        ext_step_kernel<REDUCE, KM, SAMET, true><<<grid, threads, 0, stream>>>(Tin, Tout, p);
-    else
-        ext_step_kernel<REDUCE, KM, SAMET, false><<<grid, threads, 0, stream>>>(Tin, Tout, p);
-    return cudaGetLastError();
+    return launch_chained(vec ? ext_step_kernel<REDUCE, KM, SAMET, true>
+                              : ext_step_kernel<REDUCE, KM, SAMET, false>,
+                          grid, threads, 0, stream, Tin, Tout, p);
 }
 template <bool REDUCE>
 cudaError_t launch_ext_t(bool km, int grid, const double* Tin, double* Tout, const ExtParams& p,
@@ -604,9 +615,39 @@ reduce_rows_kernel(const double* __restrict__ T, int nx, int ny, double Tm,
                    Partial* __restrict__ out) {
     const long long N = (long long)nx * ny;
     double tm = -1.0; long long ag = N; int mn = ny, mx = -1;
+    pdl_trigger();
+    pdl_wait();
     // 16-byte pairs when every row starts on a 16-byte boundary
     const bool pairs = (nx % 2 == 0) && (reinterpret_cast<uintptr_t>(T) % 16 == 0);
-    for (int y = blockIdx.x; y < ny; y += gridDim.x) {
+    // Rows shorter than the block's loads in flight: several rows at once (a
+    // row of 512 pairs alone left half the threads idle and one load per
+    // thread in flight: 8.5 us at 1024^2 for 8 MB that sit in L2).
+    const int rpp = pairs ? RR_THREADS * RR_VEC / (nx / 2) : 0;      // rows per pass
+    if (rpp > 1) {
+        const int np = nx / 2, slots = rpp * np;
+        for (long long y0 = blockIdx.x; y0 < ny; y0 += (long long)gridDim.x * rpp) {
+            double2 v[RR_VEC];
+            long long i[RR_VEC];
+            int yy[RR_VEC];
+#pragma unroll
+            for (int u = 0; u < RR_VEC; ++u) {
+                const int q = threadIdx.x + u * RR_THREADS, rr = q / np;
+                const long long y = y0 + (long long)rr * gridDim.x;
+                v[u] = make_double2(-INFINITY, -INFINITY);
+                i[u] = y * nx + 2ll * (q - rr * np);
+                yy[u] = (int)y;
+                if (q < slots && y < ny) v[u] = __ldg(reinterpret_cast<const double2*>(T + i[u]));
+            }
+#pragma unroll
+            for (int u = 0; u < RR_VEC; ++u) {
+                bool molten = false;
+                rr_take(v[u].x, i[u], tm, ag, molten, Tm);
+                rr_take(v[u].y, i[u] + 1, tm, ag, molten, Tm);
+                if (molten) { mn = min(mn, yy[u]); mx = max(mx, yy[u]); }
+            }
+        }
+    }
+    for (int y = rpp > 1 ? ny : blockIdx.x; y < ny; y += gridDim.x) {
         const double* row = T + (size_t)y * nx;
         const long long base = (long long)y * nx;
         bool molten = false;
@@ -664,6 +705,8 @@ __global__ void finalize_cluster_kernel(const Partial* __restrict__ parts, int n
     const long long N = (long long)nx * ny;
     double tm = -1.0; long long ag = N; int mn = ny, mx = -1;
     const int rank = (int)cluster.block_rank();
+    pdl_trigger();
+    pdl_wait();
     for (int i = rank * FIN_THREADS + threadIdx.x; i < nblocks; i += FIN_CTAS * FIN_THREADS) {
         const Partial q = parts[i];
         partial_take(tm, ag, mn, mx, q.tmax, q.arg, q.ymin, q.ymax);
@@ -689,9 +732,34 @@ __global__ void finalize_cluster_kernel(const Partial* __restrict__ parts, int n
     cluster.sync();   // keep every CTA's shared memory alive until rank 0 has read it
 }
 
+__global__ void __launch_bounds__(FIN_THREADS)
+finalize_small_kernel(const Partial* __restrict__ parts, int nblocks, int nx, int ny,
+                      Partial* __restrict__ out) {
+    __shared__ Partial red[FIN_THREADS / 32];
+    const long long N = (long long)nx * ny;
+    double tm = -1.0; long long ag = N; int mn = ny, mx = -1;
+    pdl_trigger();
+    pdl_wait();
+    if ((int)threadIdx.x < nblocks) {
+        const Partial q = parts[threadIdx.x];
+        partial_take(tm, ag, mn, mx, q.tmax, q.arg, q.ymin, q.ymax);
+    }
+    partial_warp_reduce(tm, ag, mn, mx);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = Partial{tm, ag, mn, mx};
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a = -1.0; long long b = N; int c = ny, d = -1;
+        for (int w = 0; w < (int)blockDim.x / 32; ++w)
+            partial_take(a, b, c, d, red[w].tmax, red[w].arg, red[w].ymin, red[w].ymax);
+        out[0] = Partial{a, b, c, d};
+    }
+}
+
 __global__ void extract_col_kernel(const double* __restrict__ T, int nx, int ny,
                                    const Partial* __restrict__ glob, double* __restrict__ col) {
     const int y = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_trigger();
+    pdl_wait();
     if (y >= ny) return;
     const long long a = glob->arg;
     const int x = (int)(a % nx);
@@ -718,7 +786,7 @@ void lpbf_launch_step(const double* Tin, double* Tout, const StepConst* k, int p
 void lpbf_launch_reduce(const double* T, int nx, int ny, double Tm, Partial* out,
                         int nblocks, cudaStream_t stream) {
     if (nblocks <= 0) return;
-    reduce_rows_kernel<<<nblocks, RR_THREADS, 0, stream>>>(T, nx, ny, Tm, out);
+    launch_chained(reduce_rows_kernel, nblocks, RR_THREADS, 0, stream, T, nx, ny, Tm, out);
 }
 
 void lpbf_launch_step_reduce(const double* Tin, double* Tout, const StepConst* k, int phys,
@@ -741,7 +809,7 @@ void lpbf_launch_reduce_finalize(const Partial* parts, int nblocks, int nx, int 
 void lpbf_launch_extract_col(const double* T, int nx, int ny, const Partial* glob,
                              double* out_col, cudaStream_t stream) {
     const int bs = 128;
-    extract_col_kernel<<<(ny + bs - 1) / bs, bs, 0, stream>>>(T, nx, ny, glob, out_col);
+    launch_chained(extract_col_kernel, (ny + bs - 1) / bs, bs, 0, stream, T, nx, ny, glob, out_col);
 }
 
 }  // extern "C"

@@ -175,6 +175,17 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     }
     return true;
 }
+// Programmatic dependent launch.  Kernels of a run are launched with
+// launch_chained (lpbf_host.hpp): the next launch's blocks may take the places
+// of finished blocks before this kernel ends.  pdl_trigger allows that;
+// pdl_wait, before a kernel's first access to global memory, waits until every
+// earlier kernel of the stream has completed and its writes are visible.
+__device__ __forceinline__ void pdl_trigger() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 // 2D tiled TMA load of box (x, y) into this CTA's shared memory.  x must be
 // even for f64 (16-byte rule); y may be negative or past the end (zero fill).
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y,

@@ -113,8 +113,7 @@ cudaError_t launch_fk(const float* hi_in, const float* lo_in, float* hi_out, flo
     } else {
         ml = mh;     // not read by the plain kernel
     }
-    kern<<<grid, ADV_WARPS * 32, smem, stream>>>(mh, ml, p);
-    return cudaGetLastError();
+    return launch_chained(kern, grid, ADV_WARPS * 32, smem, stream, mh, ml, p);
 }
 
 template <bool COMP>

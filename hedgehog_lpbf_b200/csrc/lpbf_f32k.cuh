@@ -817,6 +817,8 @@ advance_f32k_kernel(const __grid_constant__ CUtensorMap map_hi,
 
     FkStrip<K, REDUCE, SQ, COMP> ws(p, &map_hi, &map_lo, stages, bars, lane, s_tmx[wid], s_arg[wid],
                           s_ymn[wid], s_ymx[wid], s_box[wid]);
+    pdl_trigger();
+    pdl_wait();
     for (;;) {
         unsigned int t = 0;
         if (lane == 0) t = atomicAdd(p.tasks, 1u);

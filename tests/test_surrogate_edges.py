@@ -2,7 +2,9 @@
 """Gradients of the super-stepper at the edges of the narrow layers' tiles
 (128-pixel column tiles, 8-row units, 64-pixel tiles of the input gradient)
 against the FP64 restatement.  Per layer: within 3 % in norm (bf16 operands:
-the bar of the gradient tests); the loss within 1 %."""
+the bar of the gradient tests); the loss within 1 %.  The output layer's bias
+gradient is one sum of residuals that may nearly cancel, so its bar is 3 % of
+the sum of their magnitudes."""
 import numpy as np
 import pytest
 
@@ -25,12 +27,14 @@ def test_gradients_at_tile_edges(gpu, B, H, W):
     loss = float(net.gradients(x.cuda().contiguous(), torch.tensor(y).cuda()).item())
     got = S.unflatten(net.grads_vector())
     want_loss, want = R.loss_and_grads(ps, x.double().numpy(), y.astype(np.float64))
+    terms = np.sum(np.abs(2.0 / y.size * (R.forward(ps, x.double().numpy())[0] - y)))
     assert net.error_word() == 0
     assert abs(loss - want_loss) <= 1e-2 * want_loss
-    for (gw, gb), (rw, rb) in zip(got, want):
+    for i, ((gw, gb), (rw, rb)) in enumerate(zip(got, want)):
         for g, r in ((gw, rw), (gb, rb)):
             g, r = np.asarray(g).ravel(), np.asarray(r).ravel()
-            assert np.linalg.norm(g - r) <= 3e-2 * np.linalg.norm(r) + 1e-7
+            size = terms if i == 4 and r.size == 1 else np.linalg.norm(r)
+            assert np.linalg.norm(g - r) <= 3e-2 * size + 1e-7
 
 
 def test_features_in_and_around_the_source_box(gpu):
