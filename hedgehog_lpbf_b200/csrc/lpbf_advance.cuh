@@ -969,8 +969,8 @@ advance_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ 
         for (int t = 0; t < K; ++t) {
             double tm = s_red[wid].tmx[t][lane];
             long long ag = s_red[wid].arg[t][lane];
-            int mn = s_red[wid].ymn[t], mx = s_red[wid].ymx[t];
-            partial_warp_reduce(tm, ag, mn, mx);
+            const int mn = s_red[wid].ymn[t], mx = s_red[wid].ymx[t];
+            partial_warp_peak(tm, ag);
             if (lane == 0) red[wid][t] = Partial{tm, ag, mn, mx};
         }
         __syncthreads();
@@ -993,14 +993,13 @@ advance_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ 
         }
     }
     if (!p.counter) return;
-    // Last CTA: finalize the per-step Partials and re-arm the counters.
-    __threadfence();
+    // Last CTA: finalize the per-step Partials and re-arm the counters.  The
+    // ticket orders the CTA's few records only (the field's rows need no
+    // fence: the kernel's end publishes them).
     __syncthreads();
-    if (threadIdx.x == 0)
-        s_last = (atomicAdd(p.counter, 1u) == gridDim.x - 1) ? 1u : 0u;
+    if (threadIdx.x == 0) s_last = (ticket(p.counter) == gridDim.x - 1) ? 1u : 0u;
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
     if constexpr (REDUCE) {
         if (p.ring) {
             // The whole GPU waits on this CTA: every thread issues the loads
@@ -1038,7 +1037,7 @@ advance_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ 
             __syncthreads();
 #pragma unroll
             for (int t = 0; t < K; ++t) {
-                partial_warp_reduce(tm[t], ag[t], mn[t], mx[t]);
+                partial_warp_all(tm[t], ag[t], mn[t], mx[t]);
                 if (lane == 0) red[wid][t] = Partial{tm[t], ag[t], mn[t], mx[t]};
             }
             __syncthreads();

@@ -69,10 +69,11 @@ __device__ __forceinline__ void fold(const BatchLaunch& L, int s, int i, int bas
     const int ng = __ldg(&L.group_base[s + 1]) - gb;
     const long long N = (long long)nx * ny;
     unsigned int last = 0;
-    if (lane == 0) {
-        __threadfence();
-        last = (atomicAdd(&L.group_done[gb + g], 1u) == (unsigned int)(gsz - 1)) ? 1u : 0u;
-    }
+    // lane 0 wrote the task's Partials and no field cell (it is halo): the
+    // ticket's release waits for those few stores only, where a fence in every
+    // task would wait for the warp's last rows to reach memory
+    if (lane == 0)
+        last = (ticket(&L.group_done[gb + g]) == (unsigned int)(gsz - 1)) ? 1u : 0u;
     if (!__shfl_sync(0xffffffffu, last, 0)) return;
     __threadfence();
 #pragma unroll
@@ -223,8 +224,8 @@ batch_kernel(const __grid_constant__ BatchLaunch L) {
         for (int t = 0; t < K; ++t) {
             double tm = s_red[wid].tmx[t][lane];
             long long ag = s_red[wid].arg[t][lane];
-            int mn = s_red[wid].ymn[t], mx = s_red[wid].ymx[t];
-            partial_warp_reduce(tm, ag, mn, mx);
+            const int mn = s_red[wid].ymn[t], mx = s_red[wid].ymx[t];
+            partial_warp_peak(tm, ag);
             if (lane == 0) L.parts[(size_t)c_tq * K + t] = Partial{tm, ag, mn, mx};
         }
         fold<K>(L, c_s, c_tq - c_base, c_base, c_nt, par.c.nx, par.c.ny, L.scen[c_s].ring, lane);

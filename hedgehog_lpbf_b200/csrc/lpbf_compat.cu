@@ -493,13 +493,10 @@ ext_step_kernel(const double* __restrict__ Tin, double* __restrict__ Tout,
                 p.ref_out[i] = neutral;
             return;
         }
-        __threadfence();
         __syncthreads();
-        if (threadIdx.x == 0)
-            s_last = (atomicAdd(p.counter, 1u) == gridDim.x - 1) ? 1u : 0u;
+        if (threadIdx.x == 0) s_last = (ticket(p.counter) == gridDim.x - 1) ? 1u : 0u;
         __syncthreads();
         if (!s_last) return;
-        __threadfence();
         double a = -1.0; long long b = N; int c1 = ny, d1 = -1;
         for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
             const Partial* qq = &p.scratch[i];

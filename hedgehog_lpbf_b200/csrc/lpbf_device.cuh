@@ -137,6 +137,48 @@ __device__ __forceinline__ void partial_warp_reduce(double& tm, long long& ag, i
     }
 }
 
+// Order-preserving unsigned key of a double (not NaN) and back.
+__device__ __forceinline__ unsigned long long order_key(double v) {
+    const long long b = __double_as_longlong(v);
+    return (unsigned long long)b ^ ((unsigned long long)(b >> 63) | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double order_unkey(unsigned long long k) {
+    const unsigned long long b =
+        (k & 0x8000000000000000ull) ? k ^ 0x8000000000000000ull : ~k;
+    return __longlong_as_double((long long)b);
+}
+// Largest tm over the warp and the smallest index among the lanes that hold
+// it, in every lane: four integer warp reductions on the halves of the two
+// words (five rounds of shuffles take thirty).  Peaks are never NaN and
+// indices never negative.
+__device__ __forceinline__ void partial_warp_peak(double& tm, long long& ag) {
+    const unsigned long long k = order_key(tm);
+    const unsigned int hi = (unsigned int)(k >> 32), lo = (unsigned int)k;
+    const unsigned int h = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned int l = __reduce_max_sync(0xffffffffu, hi == h ? lo : 0u);
+    const bool top = hi == h && lo == l;
+    const unsigned int ah = (unsigned int)((unsigned long long)ag >> 32), al = (unsigned int)ag;
+    const unsigned int gh = __reduce_min_sync(0xffffffffu, top ? ah : 0xffffffffu);
+    const unsigned int gl = __reduce_min_sync(0xffffffffu, top && ah == gh ? al : 0xffffffffu);
+    tm = order_unkey(((unsigned long long)h << 32) | l);
+    ag = (long long)(((unsigned long long)gh << 32) | gl);
+}
+
+// The whole warp's Partial, in every lane.
+__device__ __forceinline__ void partial_warp_all(double& tm, long long& ag, int& mn, int& mx) {
+    partial_warp_peak(tm, ag);
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+}
+// Take a ticket after this thread's earlier writes, and (the release is
+// cumulative) those of threads it has synchronized with; whoever draws the
+// last one sees the writes behind the others.
+__device__ __forceinline__ unsigned int ticket(unsigned int* p) {
+    unsigned int v;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // ---- PTX: shared-memory addresses, mbarriers, TMA ----------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));

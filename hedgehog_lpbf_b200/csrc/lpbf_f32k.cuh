@@ -834,8 +834,8 @@ advance_f32k_kernel(const __grid_constant__ CUtensorMap map_hi,
         for (int t = 0; t < K; ++t) {
             double tm = s_tmx[wid][t][lane];
             long long ag = s_arg[wid][t][lane];
-            int mn = s_ymn[wid][t], mx = s_ymx[wid][t];
-            partial_warp_reduce(tm, ag, mn, mx);
+            const int mn = s_ymn[wid][t], mx = s_ymx[wid][t];
+            partial_warp_peak(tm, ag);
             if (lane == 0) red[wid][t] = Partial{tm, ag, mn, mx};
         }
         __syncthreads();
@@ -848,31 +848,50 @@ advance_f32k_kernel(const __grid_constant__ CUtensorMap map_hi,
             p.scratch[(size_t)blockIdx.x * K + t] = Partial{tm, ag, mn, mx};
         }
     }
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = (atomicAdd(p.counter, 1u) == gridDim.x - 1) ? 1u : 0u;
+    if (threadIdx.x == 0) s_last = (ticket(p.counter) == gridDim.x - 1) ? 1u : 0u;
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
     if constexpr (REDUCE) {
+        // all of a thread's record loads before any combine, as the FP64 kernel
+        constexpr int FIN_U = 5;
+        double tm[K]; long long ag[K]; int mn[K], mx[K];
+#pragma unroll
+        for (int t = 0; t < K; ++t) { tm[t] = -1.0; ag[t] = N; mn[t] = p.c.ny; mx[t] = -1; }
+        for (int i0 = threadIdx.x; i0 < (int)gridDim.x; i0 += blockDim.x * FIN_U) {
+#pragma unroll
+            for (int t = 0; t < K; ++t) {
+                Partial q[FIN_U];
+#pragma unroll
+                for (int u = 0; u < FIN_U; ++u) {
+                    const int i = i0 + u * (int)blockDim.x;
+                    q[u] = Partial{-1.0, N, p.c.ny, -1};
+                    if (i < (int)gridDim.x) {
+                        const Partial* r = &p.scratch[(size_t)i * K + t];
+                        q[u] = Partial{__ldcg(&r->tmax), __ldcg(&r->arg), __ldcg(&r->ymin),
+                                       __ldcg(&r->ymax)};
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < FIN_U; ++u)
+                    partial_take(tm[t], ag[t], mn[t], mx[t], q[u].tmax, q[u].arg, q[u].ymin,
+                                 q[u].ymax);
+            }
+        }
+        __syncthreads();
+#pragma unroll
         for (int t = 0; t < K; ++t) {
-            double tm = -1.0; long long ag = N; int mn = p.c.ny, mx = -1;
-            for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
-                const Partial* q = &p.scratch[(size_t)i * K + t];
-                partial_take(tm, ag, mn, mx, __ldcg(&q->tmax), __ldcg(&q->arg),
-                             __ldcg(&q->ymin), __ldcg(&q->ymax));
-            }
-            partial_warp_reduce(tm, ag, mn, mx);
-            __syncthreads();
-            if (lane == 0) red[wid][0] = Partial{tm, ag, mn, mx};
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double a = -1.0; long long b = N; int c1 = p.c.ny, d1 = -1;
-                for (int w = 0; w < ADV_WARPS; ++w)
-                    partial_take(a, b, c1, d1, red[w][0].tmax, red[w][0].arg,
-                                 red[w][0].ymin, red[w][0].ymax);
-                p.ring[t] = Partial{a, b, c1, d1};
-            }
+            partial_warp_all(tm[t], ag[t], mn[t], mx[t]);
+            if (lane == 0) red[wid][t] = Partial{tm[t], ag[t], mn[t], mx[t]};
+        }
+        __syncthreads();
+        if (threadIdx.x < K) {
+            const int t = threadIdx.x;
+            double a = -1.0; long long b = N; int c1 = p.c.ny, d1 = -1;
+            for (int w = 0; w < ADV_WARPS; ++w)
+                partial_take(a, b, c1, d1, red[w][t].tmax, red[w][t].arg, red[w][t].ymin,
+                             red[w][t].ymax);
+            p.ring[t] = Partial{a, b, c1, d1};
         }
     }
     if (threadIdx.x == 0) { *p.counter = 0u; *p.tasks = 0u; }

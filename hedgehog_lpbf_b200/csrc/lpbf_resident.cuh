@@ -91,16 +91,6 @@ __host__ __device__ inline int res_bound(int i, int n, int len, int unit) {
 __host__ __device__ inline int res_step(int b, int nblocks, int n) {
     return b * n / nblocks;       // n <= RES_STEPS
 }
-// Order-preserving unsigned key of a double (not NaN) and back.
-__device__ __forceinline__ unsigned long long res_key(double v) {
-    const long long b = __double_as_longlong(v);
-    return (unsigned long long)b ^ ((unsigned long long)(b >> 63) | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double res_unkey(unsigned long long k) {
-    const unsigned long long b =
-        (k & 0x8000000000000000ull) ? k ^ 0x8000000000000000ull : ~k;
-    return __longlong_as_double((long long)b);
-}
 // Largest (hi, lo) over the warp and the smallest key among the lanes that
 // hold it.
 __device__ __forceinline__ void res_warp_max(unsigned int& hi, unsigned int& lo,
@@ -469,7 +459,7 @@ resident_kernel(const __grid_constant__ ResParams p) {
                     m = g ? mj : m;
                     key = g ? kj : key;
                 }
-                const unsigned long long k64 = res_key(m);
+                const unsigned long long k64 = order_key(m);
                 unsigned int hi = (unsigned int)(k64 >> 32), lo = (unsigned int)k64;
                 res_warp_max(hi, lo, key);
                 if (lane == 0) {
@@ -478,7 +468,7 @@ resident_kernel(const __grid_constant__ ResParams p) {
                     const int col = (int)(key & ((1u << RES_KEY_SHIFT) - 1u)) + px0;
                     const int mx = s_mx[t];
                     Partial out;
-                    out.tmax = res_unkey(((unsigned long long)hi << 32) | lo);
+                    out.tmax = order_unkey(((unsigned long long)hi << 32) | lo);
                     out.arg = none ? (long long)nx * ny : (long long)row * nx + col;
                     out.ymin = mx < 0 ? ny : s_mn[t];
                     out.ymax = mx;
