@@ -306,19 +306,15 @@ using namespace lpbf_b200;
 
 namespace {
 
-// Measured on B200 at 8192^2 with the per-step reduction: depth 3 is the
-// fastest (depth 4 is register-bound); small grids fit in L2 and gain little.
-int auto_depth(int nx, int ny) {
-    const long long n = (long long)nx * ny;
-    if (n >= (1ll << 22)) return 3;
-    if (n >= (1ll << 18)) return 2;
-    return 1;
-}
+// Launch path, measured on B200 with the per-step reduction (us per step at
+// depths 1-4): 240^2 17.7, 14.9, 14.6, 17.1; 1000^2 16.2, 14.0, 12.7, 13.7;
+// 1600^2 19.2, 16.7, 15.3, 16.7; 2048^2 23.0, 18.0, 16.8, 18.9 (depth 4 is
+// register-bound).
+constexpr int AUTO_DEPTH = 3;
 
-int resolve_depth(const lpbf_b200_opts* o, int nx, int ny) {
+int resolve_depth(const lpbf_b200_opts* o) {
     if (o->phys != 0) return 1;
-    int d = o->depth > 0 ? o->depth : auto_depth(nx, ny);
-    return std::min(std::max(d, 1), 4);
+    return o->depth > 0 ? std::min(o->depth, 4) : AUTO_DEPTH;
 }
 
 // The resident kernel runs every field whose tiles fit (up to about 1.9 M
@@ -366,7 +362,7 @@ int lpbf_b200_advance_launches(int nx, int ny, int n_steps, const lpbf_b200_opts
     if (!opts || n_steps < 0) return LPBF_ERR_ARG;
     ResPlan pl;
     if (resident(opts, nx, ny, n_steps, &pl)) return (n_steps + pl.steps - 1) / pl.steps;
-    const int d = resolve_depth(opts, nx, ny);
+    const int d = resolve_depth(opts);
     return (n_steps + d - 1) / d;
 }
 
@@ -386,7 +382,7 @@ int lpbf_b200_advance(double* T_a, double* T_b, const StepConst* k, const lpbf_t
     Workspace* ws = static_cast<Workspace*>(work);
     if (ring && (!ws || work_bytes < sizeof(Workspace))) return LPBF_ERR_WORKSPACE;
 
-    const int depth = resolve_depth(opts, k->nx, k->ny);
+    const int depth = resolve_depth(opts);
     const Coef c = make_coef(*k, opts->bc, opts->T_edge, opts->Tm);
     double* cur = T_a;
     double* nxt = T_b;

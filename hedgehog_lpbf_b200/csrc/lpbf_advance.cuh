@@ -233,10 +233,9 @@ static_assert(offsetof(RedSmem<3>, box) % 16 == 0 && sizeof(RedSmem<3>) % 16 == 
 
 // TMA: rows are staged in shared memory by the copy engine (otherwise each
 // lane loads its cells directly).  BULK: the staging copies are plain bulk
-// copies, one per row, instead of tensor-map loads: no descriptor is read per
-// copy, which matters when warps work on many different fields at once (a
-// tensor map in global memory is fetched by the copy engine); requires an
-// even row length and a 16-byte aligned field.
+// copies, one per row, instead of tensor-map loads (no descriptor is read, but
+// one thread issues three copies per box instead of one); requires an even
+// row length and a 16-byte aligned field.
 // SQM: which cell_net form the strip uses — 0 the general one, 1 the
 // square-cell one, 2 the field's own (h.sq), chosen per task (the batched
 // kernel, whose fields differ).

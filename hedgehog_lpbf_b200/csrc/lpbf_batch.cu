@@ -15,9 +15,9 @@
 //    over the per-scenario task offsets, copies that scenario's launch
 //    parameters (a few hundred bytes) into its shared-memory slot and runs
 //    the same WarpStrip as the single-field kernel.  Rows are staged either
-//    by plain bulk copies (cp.async.bulk, one per row) or by tiled tensor-map
-//    loads from per-scenario maps in the workspace; bulk copies read no
-//    descriptor, which matters with hundreds of fields in flight.  Each
+//    by tiled tensor-map loads from per-scenario maps in the workspace (one
+//    copy per box) or by plain bulk copies (cp.async.bulk, one per row, which
+//    read no descriptor).  Each
 //    scenario's rows per task come from its size class (autotuned).
 //  * Per-step results.  A warp carries its lane peaks across consecutive
 //    tasks of one field (so its thresholds stay warm); after each task it
@@ -341,7 +341,10 @@ namespace {
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 int resolve_rows(const lpbf_b200_batch_opts& o, int cls, int K, int ny) {
-    int H = o.rows[cls] > 0 ? o.rows[cls] : 24;
+    // Automatic: GCell-updates/s at depth 3 against 24 rows throughout: 256
+    // mixed fields 467 : 339, 64 406 : 322, 12 242 : 206; 200 of 1024^2 386 : 329.
+    constexpr int AUTO_ROWS[4] = {24, 24, 48, 96};
+    int H = o.rows[cls] > 0 ? o.rows[cls] : AUTO_ROWS[cls];
     H = std::max(H, std::max(8, 4 * K));
     return std::min(H, ny);
 }
@@ -620,13 +623,22 @@ int lpbf_b200_batch_create(const lpbf_b200_scenario* sc, int n_scen, int n_steps
 
     // Staged loads need even rows and 16-byte aligned fields; one field
     // without them switches the batch to direct loads.  Automatic staging:
-    // bulk row copies, unless the batch holds few fields (then one tensor
-    // map per buffer stays resident in the copy engine's descriptor cache).
+    // tensor maps, one copy per box issued by one thread instead of one per
+    // row (GCell-updates/s against bulk row copies at depth 2: 12 mixed fields
+    // 251 : 239, 64 445 : 413, 256 537 : 495; 200 of 1024^2 496 : 463; 256 of
+    // 256^2 88 : 84), bulk copies if a map cannot be encoded.
     bool can_stage = true;
     for (int i = 0; i < n_scen; ++i)
         can_stage = can_stage && tma_ok(sc[i].T_a, sc[i].k->nx) && tma_ok(sc[i].T_b, sc[i].k->nx);
-    int stage = o.staging == 0 ? (n_scen <= 4 ? BATCH_STAGE_TMAP : BATCH_STAGE_BULK) : o.staging;
+    int stage = o.staging == 0 ? BATCH_STAGE_TMAP : o.staging;
     if (!can_stage) stage = BATCH_STAGE_DIRECT;
+    if (stage == BATCH_STAGE_TMAP && o.staging == 0) {
+        CUtensorMap probe;
+        for (int i = 0; i < n_scen && stage == BATCH_STAGE_TMAP; ++i)
+            for (double* t : {sc[i].T_a, sc[i].T_b})
+                if (!tensor_map_f64(t, sc[i].k->nx, sc[i].k->ny, ADV_COLS, ADV_R, &probe))
+                    stage = BATCH_STAGE_BULK;
+    }
 
     // Warm the per-device occupancy cache now: a later run may be captured
     // into a graph, where these queries are best avoided.

@@ -77,11 +77,7 @@ extern "C" int lpbf_b200_advance_noalloc(double* T_a, double* T_b, const StepCon
     const size_t N = (size_t)k->nx * k->ny;
     if (T_a < T_b + N && T_b < T_a + N) return LPBF_ERR_ARG;
 
-    int depth = opts->depth;
-    if (depth <= 0) {
-        const long long n = (long long)k->nx * k->ny;
-        depth = (n >= (1ll << 22)) ? 3 : (n >= (1ll << 18)) ? 2 : 1;
-    }
+    int depth = opts->depth > 0 ? opts->depth : 3;       // as lpbf_b200_advance's launch path
     depth = std::min(std::max(depth, 1), 4);
 
     void* scratch = nullptr;

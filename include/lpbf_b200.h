@@ -215,9 +215,10 @@ typedef struct lpbf_b200_scenario {
 typedef struct lpbf_b200_batch_opts {
     int depth;              /* time steps per launch, 1..4; 0 = 3 */
     int ctas_per_sm;        /* CTAs per SM of the persistent grid; 0 = as many as fit */
-    int rows[4];            /* rows per task by size class (lpbf_b200_batch_size_class); 0 = 24 */
+    int rows[4];            /* rows per task by size class (lpbf_b200_batch_size_class);
+                             * 0 = 24, 24, 48, 96 */
     int staging;            /* rows into shared memory by 1 bulk row copies, 2 per-field tensor
-                               maps; 0 = automatic (maps for <= 4 fields, else bulk copies);
+                               maps; 0 = automatic (maps, or bulk copies if none can be made);
                                fields with odd nx or 16-byte misalignment use direct loads */
 } lpbf_b200_batch_opts;
 
