@@ -43,6 +43,7 @@ struct ConvArgs {
     void* out;              // GELU/DGELU: bf16 [P][N]; LINEAR: fp32 [P]
     int B, H, W;
     unsigned int* err;
+    int run;                // row-streaming forms: output rows per work unit
     int wide;               // activations on 32-byte boundaries: 256-bit accesses
 };
 
@@ -494,7 +495,7 @@ constexpr int CR_RAW_BYTES = CR_RAW_PAIRS * 16;   // loaded per 4-channel row
 constexpr int CR_RAW_PITCH = 1152;                 // raw slot pitch
 constexpr int CR_RAW = 4;                          // raw 4-channel row slots
 constexpr int CR_SLOTS = 5;                        // operand slots
-constexpr int CR_RUN = 32;                         // output rows per work unit
+constexpr int CR_RUN = 32;                         // most output rows per work unit
 constexpr int CR_CTAS = 3;                         // CTAs per SM
 constexpr int CR_NACC = 2;                         // TMEM accumulators
 // a TMA tensor copy lands on a 128-byte boundary
@@ -511,31 +512,40 @@ constexpr size_t cr_smem_bytes() {
 
 // Work unit u: column tile xt, image b, output rows y0 .. y0 + n - 1.
 struct RowUnit { int b, xt, y0, n; };
-__device__ __forceinline__ RowUnit row_unit(int u, int xtiles, int runs, int H) {
+__device__ __forceinline__ RowUnit row_unit(int u, int xtiles, int runs, int H, int run) {
     RowUnit r;
     r.xt = u % xtiles;
     const int t = u / xtiles;
     r.b = t / runs;
-    r.y0 = (t % runs) * CR_RUN;
-    r.n = min(CR_RUN, H - r.y0);
+    r.y0 = (t % runs) * run;
+    r.n = min(run, H - r.y0);
     return r;
+}
+// Rows per unit (ConvArgs::run): CR_RUN, or fewer where the image would leave
+// CTAs without a unit (a unit's rows follow one another: a 167 x 70 image in
+// six 32-row units took 24 us per layer).
+inline int row_run(int B, int H, int xtiles) {
+    const long long want = (long long)CR_CTAS * sm_count();
+    int run = CR_RUN;
+    while (run > 4 && (long long)xtiles * B * ((H + run - 1) / run) < want) run /= 2;
+    return run;
 }
 
 // The input rows of a CTA's units in order: unit u, row L = 0 .. n + 1
 // (field row y0 - 1 + L).
 struct RowCursor {
-    int u, L, nunits, xtiles, runs, H;
+    int u, L, nunits, xtiles, runs, H, run;
     RowUnit r;
-    __device__ RowCursor(int u0, int nu, int xt, int ru, int h)
-        : u(u0), L(0), nunits(nu), xtiles(xt), runs(ru), H(h) {
-        if (u < nunits) r = row_unit(u, xtiles, runs, H);
+    __device__ RowCursor(int u0, int nu, int xt, int ru, int h, int rn)
+        : u(u0), L(0), nunits(nu), xtiles(xt), runs(ru), H(h), run(rn) {
+        if (u < nunits) r = row_unit(u, xtiles, runs, H, run);
     }
     __device__ bool valid() const { return u < nunits; }
     __device__ void next() {
         if (++L == r.n + 2) {
             L = 0;
             u += gridDim.x;
-            if (u < nunits) r = row_unit(u, xtiles, runs, H);
+            if (u < nunits) r = row_unit(u, xtiles, runs, H, run);
         }
     }
 };
@@ -614,7 +624,7 @@ conv_row_kernel(const __grid_constant__ CUtensorMap xmap, const ConvArgs a, int 
         if constexpr (CIN == 32) {
             if (lane == 0) {
                 uint32_t g = 0;                      // input rows issued
-                for (RowCursor c(blockIdx.x, nunits, xtiles, runs, a.H); c.valid(); c.next(), ++g) {
+                for (RowCursor c(blockIdx.x, nunits, xtiles, runs, a.H, a.run); c.valid(); c.next(), ++g) {
                     const uint32_t s = g % S;
                     if (!mbar_wait_bounded(&empty[s], ((g / S) & 1) ^ 1)) { ok = false; break; }
                     mbar_expect_tx(&full[s], CR_ROW_BYTES);
@@ -628,7 +638,7 @@ conv_row_kernel(const __grid_constant__ CUtensorMap xmap, const ConvArgs a, int 
                 }
             }
         } else {
-            RowCursor c(blockIdx.x, nunits, xtiles, runs, a.H);
+            RowCursor c(blockIdx.x, nunits, xtiles, runs, a.H, a.run);
             uint32_t issued = 0, g = 0;
             auto issue = [&]() {                     // next raw row into its slot
                 if (lane == 0) {
@@ -694,7 +704,7 @@ conv_row_kernel(const __grid_constant__ CUtensorMap xmap, const ConvArgs a, int 
             make_tensor(make_smem_ptr(reinterpret_cast<bf16*>(sB)), LayRowB<N>{}));
         uint32_t g = 0, o = 0;                       // first input row of the unit; outputs
         for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
-            const RowUnit r = row_unit(u, xtiles, runs, a.H);
+            const RowUnit r = row_unit(u, xtiles, runs, a.H, a.run);
             for (int j = 0; j < r.n; ++j, ++o) {
                 const int acc = o % CR_NACC;
                 bool w = mbar_wait_bounded(&tempty[acc], ((o / CR_NACC) & 1) ^ 1);
@@ -746,7 +756,7 @@ conv_row_kernel(const __grid_constant__ CUtensorMap xmap, const ConvArgs a, int 
             bias[c] = (EPI == EPI_GELU && active) ? __ldg(a.bias + 16 * h + c) : 0.0f;
         uint32_t o = 0;
         for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
-            const RowUnit r = row_unit(u, xtiles, runs, a.H);
+            const RowUnit r = row_unit(u, xtiles, runs, a.H, a.run);
             for (int j = 0; j < r.n; ++j, ++o) {
                 const int acc = o % CR_NACC;
                 const int x = r.xt * 128 + q * 32 + lane;
@@ -856,7 +866,7 @@ wgrad_row_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         if (lane == 0) {
             uint32_t gx = 0, gg = 0;                 // rows issued into each ring
             for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
-                const RowUnit r = row_unit(u, xtiles, runs, a.H);
+                const RowUnit r = row_unit(u, xtiles, runs, a.H, a.run);
                 for (int L = 0; L < r.n + 2 && ok; ++L) {
                     uint32_t s = gx % WR_XS;
                     if (!mbar_wait_bounded(&xempty[s], ((gx / WR_XS) & 1) ^ 1)) { ok = false; break; }
@@ -893,7 +903,7 @@ wgrad_row_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         uint32_t gx = 0, gg = 0;
         bool first = true;
         for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
-            const RowUnit r = row_unit(u, xtiles, runs, a.H);
+            const RowUnit r = row_unit(u, xtiles, runs, a.H, a.run);
             for (int j = 0; j < r.n; ++j, ++gg) {
                 bool w = mbar_wait_bounded(&gfull[gg % WR_GS], (gg / WR_GS) & 1);
 #pragma unroll
@@ -933,7 +943,7 @@ wgrad_row_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         float bsum = 0.0f;
         uint32_t gg = 0;
         for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
-            const RowUnit r = row_unit(u, xtiles, runs, a.H);
+            const RowUnit r = row_unit(u, xtiles, runs, a.H, a.run);
             for (int j = 0; j < r.n; ++j, ++gg) {
                 if (!__all_sync(0xffffffffu,
                                 mbar_wait_bounded(&gfull[gg % WR_GS], (gg / WR_GS) & 1))) {
@@ -1029,14 +1039,14 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* g, int B, int H, int W,
     constexpr size_t smem = 1024 + size_t(WR_XS) * CR_PITCH32 + size_t(WR_GS) * WR_GBYTES;
     if (const cudaError_t e = smem_opt_in<wgrad_row_kernel>(smem); e != cudaSuccess) return e;
     const int xtiles = (W + 127) / 128;
-    const int runs = (H + CR_RUN - 1) / CR_RUN;
+    const int run = row_run(B, H, xtiles), runs = (H + run - 1) / run;
     const long long nu = (long long)xtiles * runs * B;
     const long long P = (long long)B * H * W;
     if (nu >= (1ll << 31)) return cudaErrorInvalidValue;
     const int grid = (int)std::min<long long>(
         {nu, (long long)CR_CTAS * sm_count(), (long long)WR_MAX_CTAS, P});
     ConvArgs a{};
-    a.B = B; a.H = H; a.W = W; a.err = err;
+    a.B = B; a.H = H; a.W = W; a.err = err; a.run = run;
     wgrad_row_kernel<<<grid, CT_THREADS, smem, s>>>(xm, gm, a, partial, (int)nu, xtiles, runs);
     wgrad_row_reduce<<<(WR_REC + 31) / 32, dim3(32, 8), 0, s>>>(partial, grid, dw, db);
     return cudaGetLastError();
@@ -1485,7 +1495,7 @@ cudaError_t launch_conv_tma(const ConvArgs& a, cudaStream_t s) {
 }
 
 template <int CIN, int N, int EPI>
-cudaError_t launch_conv_row(const ConvArgs& a, cudaStream_t s) {
+cudaError_t launch_conv_row(ConvArgs a, cudaStream_t s) {
     CUtensorMap map;
     if (reinterpret_cast<uintptr_t>(a.x) % 16 != 0) return cudaErrorNotSupported;
     if (CIN == 32 ? !tensor_map_act_bf16(a.x, 32, a.W, a.H, a.B, CR_PX, &map)
@@ -1497,7 +1507,8 @@ cudaError_t launch_conv_row(const ConvArgs& a, cudaStream_t s) {
     if (const cudaError_t e = smem_opt_in<conv_row_kernel<CIN, N, EPI>>(smem); e != cudaSuccess)
         return e;
     const int xtiles = (a.W + 127) / 128;
-    const int runs = (a.H + CR_RUN - 1) / CR_RUN;
+    a.run = row_run(a.B, a.H, xtiles);
+    const int runs = (a.H + a.run - 1) / a.run;
     const long long nu = (long long)xtiles * runs * a.B;
     if (nu >= (1ll << 31)) return cudaErrorInvalidValue;
     const int grid = (int)std::min<long long>(nu, (long long)CR_CTAS * sm_count());
