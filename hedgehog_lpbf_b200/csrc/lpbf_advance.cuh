@@ -385,7 +385,10 @@ struct WarpStrip {
             }
         }
         const int jlast = y1 - 1 + K;
-        if (src_strip && y0 - K <= p.band_hi && y1 + K >= p.band_lo) fill_columns();
+        // For every task with a box that may read them (src_box below): its first
+        // box starts up to two rows above y0 - K, so a task right below the source
+        // rows (band_chunks) has one too, though only with rows of no use.
+        if (src_strip && jy0 - K <= p.band_hi && y1 + K >= p.band_lo) fill_columns();
         // per-box thresholds change only when an exact pass moves a peak
         if constexpr (REDUCE) set_thresholds();
         for (int b = 0, j = jy0; j <= jlast && !failed; ++b, j += ADV_R) {

@@ -185,7 +185,8 @@ struct FkStrip {
     const int lane;
 
     int x0, xs, xl, y0, y1, jy0, jend, nbox, issued;
-    bool edge, failed, src_strip, own_all;
+    bool edge, failed, own_all;
+    bool src_task;                     // rows the task depends on meet the source
     bool first_col, last_col;          // the lane holds the field's first / last column (mirror)
     double rowf;                       // this box's row factors of the source (as WarpStrip)
     double* colf;                      // the task's column factors, four per level
@@ -267,7 +268,10 @@ struct FkStrip {
         jend = min(y1 + K, ny);
         nbox = (jend - jy0 + ADV_R - 1) / ADV_R;
         edge = (xs <= 0) || (xs + ADV_COLS > nx - 1);
-        src_strip = !(xs + ADV_COLS <= p.bandx_lo || xs > p.bandx_hi);
+        // one condition for the column factors and for the boxes that read them:
+        // rows y0 - K .. y1 + K are all that an owned row depends on
+        src_task = !(xs + ADV_COLS <= p.bandx_lo || xs > p.bandx_hi) &&
+                   y0 - K <= p.band_hi && y1 + K >= p.band_lo;
         own_all = owned_lane();            // nx is a multiple of 4: whole lanes
         first_col = p.c.bc == 0 && xl == 0;
         last_col = p.c.bc == 0 && xl + V == nx;
@@ -277,7 +281,7 @@ struct FkStrip {
             for (int b = 0; b < pre; ++b) issue(b);
         }
         const int jlast = y1 - 1 + K;
-        if (src_strip && y0 - K <= p.band_hi && y1 + K >= p.band_lo) columns_to(colf, xl, p);
+        if (src_task) columns_to(colf, xl, p);
         // per-box thresholds change only when an exact pass moves a peak
         if constexpr (REDUCE) set_thresholds();
         for (int b = 0, j = jy0; j <= jlast && !failed; ++b, j += ADV_R) {
@@ -295,7 +299,7 @@ struct FkStrip {
             }
             // mirror-edge strips too: row_update patches the edge cells'
             // outer neighbours itself (nx a multiple of 4: whole lanes)
-            const bool src_box = src_strip && j + 1 >= p.band_lo && j - K <= p.band_hi;
+            const bool src_box = src_task && j + 1 >= p.band_lo && j - K <= p.band_hi;
             const bool fast = (!edge || (p.c.bc == 0 && (p.c.nx & 3) == 0)) &&
                               j - K >= 1 && j + 1 <= ny - 2 && j < jend;
             rowf = 0.0;
