@@ -340,7 +340,7 @@ resident_kernel(const __grid_constant__ ResParams p) {
                 if constexpr (REDUCE) {
                     // owned rows [oa, ob) of this warp
                     const int oa = max(ty0 - y, 0), ob = min(ty1 - y, NR);
-                    bool hot = false;
+                    bool hot = false, nan = false;
                     double rm[NR];
                     unsigned int rk[NR];
 #pragma unroll
@@ -358,6 +358,9 @@ resident_kernel(const __grid_constant__ ResParams p) {
                         for (int s = 1; s < V; s *= 2)
 #pragma unroll
                             for (int v = 0; v + s < V; v += 2 * s) {
+                                // a pair's left cell, NaN, has hidden the right
+                                // one; only in place 0 does it show at the end
+                                if (s > 1) nan |= isnan(w[v + s]);
                                 const bool g = w[v + s] > w[v];
                                 w[v] = g ? w[v + s] : w[v];
                                 wk[v] = g ? wk[v + s] : wk[v];
@@ -366,13 +369,13 @@ resident_kernel(const __grid_constant__ ResParams p) {
                         rk[i] = wk[0] + ((unsigned)i << RES_KEY_SHIFT);
                         hot |= !(rm[i] <= c.Tm);
                     }
-                    if (__any_sync(0xffffffffu, hot)) {
+                    if (__any_sync(0xffffffffu, hot || nan)) {
                         // a molten row, or one whose maximum met a NaN (NaN
                         // never wins: such a row is scanned again without it)
                         unsigned int rows = 0u;
 #pragma unroll
                         for (int i = 0; i < NR; ++i) {
-                            if (isnan(rm[i])) {
+                            if (isnan(rm[i]) || (nan && own_x && i >= oa && i < ob)) {
                                 rm[i] = -INFINITY;
 #pragma unroll
                                 for (int v = 0; v < V; ++v)
