@@ -62,6 +62,7 @@ constexpr int RES_FLAG_STRIDE = 8;  // flags 32 bytes apart
 static_assert(sizeof(Workspace::flags) >= RES_MAX_TILES * RES_FLAG_STRIDE * sizeof(unsigned), "flags");
 static_assert(WS_PARTS >= RES_MAX_TILES * RES_STEPS, "records");
 constexpr int RES_KEY_SHIFT = 8;    // local key of a cell: row << 8 | column (at most 128)
+constexpr unsigned int RES_NO_KEY = 0x7fffffffu;      // a lane without a peak
 constexpr unsigned long long RES_WAIT_NS = 4000000000ull;
 
 struct ResParams {
@@ -91,15 +92,19 @@ __host__ __device__ inline int res_bound(int i, int n, int len, int unit) {
 __host__ __device__ inline int res_step(int b, int nblocks, int n) {
     return b * n / nblocks;       // n <= RES_STEPS
 }
-// Largest (hi, lo) over the warp and the smallest key among the lanes that
-// hold it.
-__device__ __forceinline__ void res_warp_max(unsigned int& hi, unsigned int& lo,
-                                             unsigned int& key) {
+// Largest m over the warp and the smallest key (below 2^31) among the lanes
+// that hold it, in every lane: partial_warp_peak with short indices.
+__device__ __forceinline__ void res_warp_max(double& m, unsigned int& key) {
+    unsigned long long k = order_key(m);
+    const unsigned int z = k == NEG_ZERO_KEY ? 1u : 0u;
+    k += z;
+    const unsigned int hi = (unsigned int)(k >> 32), lo = (unsigned int)k;
     const unsigned int h = __reduce_max_sync(0xffffffffu, hi);
     const unsigned int l = __reduce_max_sync(0xffffffffu, hi == h ? lo : 0u);
-    key = __reduce_min_sync(0xffffffffu, (hi == h && lo == l) ? key : 0xffffffffu);
-    hi = h;
-    lo = l;
+    const unsigned int g =
+        __reduce_min_sync(0xffffffffu, hi == h && lo == l ? key << 1 | z : 0xffffffffu);
+    m = g & 1u ? -0.0 : order_unkey(((unsigned long long)h << 32) | l);
+    key = g >> 1;
 }
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
@@ -289,7 +294,7 @@ resident_kernel(const __grid_constant__ ResParams p) {
             // rows this step must leave valid: one less per side and step
             const int grow = kb - 1 - t;
             double m = -1.0;
-            unsigned int key = 0xffffffffu;
+            unsigned int key = RES_NO_KEY;
             if (y + NR > max(ty0 - grow, 0) && y < min(ty1 + grow, ny)) {
                 double up[V], dn[V], cf[V];
                 res_lds<V>(up, &s_seam[buf][max(wid - 1, 0)][NR > 1 ? 1 : 0][V * lane]);
@@ -452,7 +457,7 @@ resident_kernel(const __grid_constant__ ResParams p) {
             // this CTA's Partial of each step of the block, one warp per step
             for (int t = wid; t < kb; t += RES_WARPS) {
                 double m = -1.0;
-                unsigned int key = 0xffffffffu;
+                unsigned int key = RES_NO_KEY;
                 // warps hold rows in order: strict '>' keeps the first maximum
 #pragma unroll
                 for (int j = 0; j < RES_WARPS; ++j) {
@@ -462,16 +467,14 @@ resident_kernel(const __grid_constant__ ResParams p) {
                     m = g ? mj : m;
                     key = g ? kj : key;
                 }
-                const unsigned long long k64 = order_key(m);
-                unsigned int hi = (unsigned int)(k64 >> 32), lo = (unsigned int)k64;
-                res_warp_max(hi, lo, key);
+                res_warp_max(m, key);
                 if (lane == 0) {
-                    const bool none = key == 0xffffffffu;
+                    const bool none = key == RES_NO_KEY;
                     const int row = (int)(key >> RES_KEY_SHIFT) + py0;
                     const int col = (int)(key & ((1u << RES_KEY_SHIFT) - 1u)) + px0;
                     const int mx = s_mx[t];
                     Partial out;
-                    out.tmax = order_unkey(((unsigned long long)hi << 32) | lo);
+                    out.tmax = m;
                     out.arg = none ? (long long)nx * ny : (long long)row * nx + col;
                     out.ymin = mx < 0 ? ny : s_mn[t];
                     out.ymax = mx;
