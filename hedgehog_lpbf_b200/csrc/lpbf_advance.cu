@@ -399,10 +399,7 @@ int lpbf_b200_advance(double* T_a, double* T_b, const StepConst* k, const lpbf_t
             const cudaError_t e = launch_resident(pl, cur, nxt, cur, c, las, n,
                                                   ring ? ring + s0 : nullptr, ws, stream);
             // a context given fewer SMs than the device has: launch path
-            if (e == cudaErrorCooperativeLaunchTooLarge && s0 == 0) {
-                cudaGetLastError();
-                break;
-            }
+            if (e == cudaErrorCooperativeLaunchTooLarge && s0 == 0) break;
             if (e != cudaSuccess) return LPBF_ERR_CUDA;
             std::swap(cur, nxt);
             in_b ^= 1;

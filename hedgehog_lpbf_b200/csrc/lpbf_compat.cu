@@ -113,8 +113,8 @@ __global__ void finalize_small_kernel(const Partial* __restrict__ parts, int nbl
 inline cudaError_t launch_finalize(const Partial* parts, int nblocks, int nx, int ny,
                                    Partial* out, cudaStream_t stream) {
     if (nblocks <= FIN_THREADS)
-        return launch_chained(finalize_small_kernel, 1, nblocks <= 256 ? 256 : FIN_THREADS, 0,
-                              stream, parts, nblocks, nx, ny, out);
+        return launch_chained_raw(finalize_small_kernel, 1, nblocks <= 256 ? 256 : FIN_THREADS,
+                                  0, stream, parts, nblocks, nx, ny, out);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(FIN_CTAS, 1, 1);
     cfg.blockDim = dim3(FIN_THREADS, 1, 1);
@@ -783,7 +783,7 @@ void lpbf_launch_step(const double* Tin, double* Tout, const StepConst* k, int p
 void lpbf_launch_reduce(const double* T, int nx, int ny, double Tm, Partial* out,
                         int nblocks, cudaStream_t stream) {
     if (nblocks <= 0) return;
-    launch_chained(reduce_rows_kernel, nblocks, RR_THREADS, 0, stream, T, nx, ny, Tm, out);
+    launch_chained_raw(reduce_rows_kernel, nblocks, RR_THREADS, 0, stream, T, nx, ny, Tm, out);
 }
 
 void lpbf_launch_step_reduce(const double* Tin, double* Tout, const StepConst* k, int phys,
@@ -806,7 +806,8 @@ void lpbf_launch_reduce_finalize(const Partial* parts, int nblocks, int nx, int 
 void lpbf_launch_extract_col(const double* T, int nx, int ny, const Partial* glob,
                              double* out_col, cudaStream_t stream) {
     const int bs = 128;
-    launch_chained(extract_col_kernel, (ny + bs - 1) / bs, bs, 0, stream, T, nx, ny, glob, out_col);
+    launch_chained_raw(extract_col_kernel, (ny + bs - 1) / bs, bs, 0, stream, T, nx, ny, glob,
+                       out_col);
 }
 
 }  // extern "C"

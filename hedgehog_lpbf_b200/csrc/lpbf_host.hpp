@@ -63,10 +63,11 @@ bool tensor_map_act_bf16(const void* base, int C, int W, int H, int B, int box_p
 // Launch whose blocks may become resident while the stream's previous kernel
 // drains (that kernel and this one call pdl_trigger / pdl_wait): the launch
 // latency and the kernel's own set-up then hide behind the previous tail.
-// Between back-to-back short kernels it saves 2-4 us each.
+// Between back-to-back short kernels it saves 2-4 us each.  A refused launch
+// stays the runtime's last error, as after <<<>>>.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_chained(void (*kern)(KArgs...), unsigned grid, unsigned block,
-                                  size_t smem, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_chained_raw(void (*kern)(KArgs...), unsigned grid, unsigned block,
+                                      size_t smem, cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid, 1, 1);
     cfg.blockDim = dim3(block, 1, 1);
@@ -78,6 +79,16 @@ inline cudaError_t launch_chained(void (*kern)(KArgs...), unsigned grid, unsigne
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+// Where the call's own status reports a refused launch, it is not left as the
+// last error too: the next CUDA call that looks there is not this one's.
+inline cudaError_t take_error(cudaError_t e) {
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+template <typename... Args>
+inline cudaError_t launch_chained(Args&&... args) {
+    return take_error(launch_chained_raw(std::forward<Args>(args)...));
 }
 
 // Rows whose source term can be non-zero in any of the K substeps (a

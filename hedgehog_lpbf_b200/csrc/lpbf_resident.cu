@@ -35,7 +35,7 @@ cudaError_t launch_t(const ResParams& p, cudaStream_t stream) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, resident_kernel<V, NR, MODE, REDUCE>, p);
+    return take_error(cudaLaunchKernelEx(&cfg, resident_kernel<V, NR, MODE, REDUCE>, p));
 }
 
 template <int V, int NR>
