@@ -481,7 +481,7 @@ struct WarpStrip {
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 const int x = xl + v;
-                dst[v] = (x >= 0 && x < nx) ? __ldg(rowp + x) : 0.0;
+                dst[v] = (x >= 0 && x < nx) ? rowp[x] : 0.0;
             }
         }
     }

@@ -96,15 +96,15 @@ ExtLines make_ext_lines() {
     return L;
 }
 
-__global__ void reduce_rows_kernel(const double* __restrict__ T, int nx, int ny, double Tm,
-                                   Partial* __restrict__ out);
+__global__ void reduce_rows_kernel(const double* T, int nx, int ny, double Tm,
+                                   Partial* out);
 constexpr int FIN_CTAS = 8;
 constexpr int FIN_THREADS = 512;
-__global__ void finalize_cluster_kernel(const Partial* __restrict__ parts, int nblocks, int nx, int ny,
-                        Partial* __restrict__ out);
+__global__ void finalize_cluster_kernel(const Partial* parts, int nblocks, int nx, int ny,
+                        Partial* out);
 
-__global__ void finalize_small_kernel(const Partial* __restrict__ parts, int nblocks, int nx,
-                                      int ny, Partial* __restrict__ out);
+__global__ void finalize_small_kernel(const Partial* parts, int nblocks, int nx,
+                                      int ny, Partial* out);
 
 // Launch finalize_cluster_kernel as one cluster of FIN_CTAS CTAs, or, for up
 // to FIN_THREADS Partials (the unfused reduce's 256), one CTA: a cluster's
@@ -276,16 +276,16 @@ struct ExtStrip {
 // 16-byte boundaries, nx even): a pair lies wholly on or off the field; one
 // off it takes the edge cell twice.
 template <bool VEC>
-__device__ __forceinline__ void ext_load(const double* __restrict__ Tin, int nx, int ny, int y,
+__device__ __forceinline__ void ext_load(const double* Tin, int nx, int ny, int y,
                                          const ExtStrip& s, double& u, double& v) {
     const double* row = Tin + (size_t)min(max(y, 0), ny - 1) * nx;
     if constexpr (VEC) {
-        const double2 t = __ldg(reinterpret_cast<const double2*>(row + s.cv));
+        const double2 t = *reinterpret_cast<const double2*>(row + s.cv);
         u = s.xa >= nx ? t.y : t.x;
         v = s.xa < 0 ? t.x : t.y;
     } else {
-        u = __ldg(row + s.ca);
-        v = __ldg(row + s.cb);
+        u = row[s.ca];
+        v = row[s.cb];
     }
 }
 
@@ -295,8 +295,8 @@ __device__ __forceinline__ void ext_load(const double* __restrict__ Tin, int nx,
 // the reciprocal five dependent operations) overlap.  With a branch per row a
 // lone warp took 1 us per row.  SRC: the block meets the source.
 template <bool REDUCE, bool KM, bool SAMET, bool VEC, bool SRC>
-__device__ __forceinline__ void ext_block(const double* __restrict__ Tin,
-                                          double* __restrict__ Tout, const ExtParams& p,
+__device__ __forceinline__ void ext_block(const double* Tin,
+                                          double* Tout, const ExtParams& p,
                                           const ExtLines& L, int y, ExtStrip& s,
                                           double (&Q)[EXT_R][2], int lane) {
     const StepConst& k = p.k;
@@ -407,7 +407,7 @@ __device__ __forceinline__ void ext_block(const double* __restrict__ Tin,
 // the last CTA.
 template <bool REDUCE, bool KM, bool SAMET, bool VEC>
 __global__ void __launch_bounds__(EXT_WARPS * 32, 2)
-ext_step_kernel(const double* __restrict__ Tin, double* __restrict__ Tout,
+ext_step_kernel(const double* Tin, double* Tout,
                 const __grid_constant__ ExtParams p) {
     const StepConst& k = p.k;
     __shared__ ExtLines L;
@@ -607,9 +607,12 @@ __device__ __forceinline__ void rr_take(double v, long long i, double& tm, long 
     molten |= (v > Tm);
 }
 
-__global__ void __launch_bounds__(RR_THREADS)
-reduce_rows_kernel(const double* __restrict__ T, int nx, int ny, double Tm,
-                   Partial* __restrict__ out) {
+// 48 registers: a CTA then fits beside the step's last CTA on its SM and waits
+// there for the field (56, which the loads alone would take: step, reduce and
+// finalize at 1024^2 19.2 us against 18.2; at 2048^2 28.0 against 27.4).
+__global__ void __maxnreg__(48)
+reduce_rows_kernel(const double* T, int nx, int ny, double Tm,
+                   Partial* out) {
     const long long N = (long long)nx * ny;
     double tm = -1.0; long long ag = N; int mn = ny, mx = -1;
     pdl_trigger();
@@ -624,22 +627,22 @@ reduce_rows_kernel(const double* __restrict__ T, int nx, int ny, double Tm,
         const int np = nx / 2, slots = rpp * np;
         for (long long y0 = blockIdx.x; y0 < ny; y0 += (long long)gridDim.x * rpp) {
             double2 v[RR_VEC];
-            long long i[RR_VEC];
-            int yy[RR_VEC];
+            int xx[RR_VEC], yy[RR_VEC];
 #pragma unroll
             for (int u = 0; u < RR_VEC; ++u) {
                 const int q = threadIdx.x + u * RR_THREADS, rr = q / np;
                 const long long y = y0 + (long long)rr * gridDim.x;
                 v[u] = make_double2(-INFINITY, -INFINITY);
-                i[u] = y * nx + 2ll * (q - rr * np);
+                xx[u] = 2 * (q - rr * np);
                 yy[u] = (int)y;
-                if (q < slots && y < ny) v[u] = __ldg(reinterpret_cast<const double2*>(T + i[u]));
+                if (q < slots && y < ny) v[u] = *reinterpret_cast<const double2*>(T + y * nx + xx[u]);
             }
 #pragma unroll
             for (int u = 0; u < RR_VEC; ++u) {
                 bool molten = false;
-                rr_take(v[u].x, i[u], tm, ag, molten, Tm);
-                rr_take(v[u].y, i[u] + 1, tm, ag, molten, Tm);
+                const long long i = (long long)yy[u] * nx + xx[u];
+                rr_take(v[u].x, i, tm, ag, molten, Tm);
+                rr_take(v[u].y, i + 1, tm, ag, molten, Tm);
                 if (molten) { mn = min(mn, yy[u]); mx = max(mx, yy[u]); }
             }
         }
@@ -656,7 +659,7 @@ reduce_rows_kernel(const double* __restrict__ T, int nx, int ny, double Tm,
 #pragma unroll
                 for (int u = 0; u < RR_VEC; ++u) {
                     const int p = p0 + u * RR_THREADS;
-                    v[u] = p < np ? __ldg(r2 + p) : make_double2(-INFINITY, -INFINITY);
+                    v[u] = p < np ? r2[p] : make_double2(-INFINITY, -INFINITY);
                 }
 #pragma unroll
                 for (int u = 0; u < RR_VEC; ++u) {
@@ -671,7 +674,7 @@ reduce_rows_kernel(const double* __restrict__ T, int nx, int ny, double Tm,
 #pragma unroll
                 for (int u = 0; u < RR_VEC; ++u) {
                     const int x = x0 + u * RR_THREADS;
-                    v[u] = x < nx ? __ldg(row + x) : -INFINITY;
+                    v[u] = x < nx ? row[x] : -INFINITY;
                 }
 #pragma unroll
                 for (int u = 0; u < RR_VEC; ++u)
@@ -694,8 +697,8 @@ reduce_rows_kernel(const double* __restrict__ T, int nx, int ny, double Tm,
 
 // ---- finalize: one cluster of FIN_CTAS CTAs ----------------------------------
 
-__global__ void finalize_cluster_kernel(const Partial* __restrict__ parts, int nblocks, int nx, int ny,
-                        Partial* __restrict__ out) {
+__global__ void finalize_cluster_kernel(const Partial* parts, int nblocks, int nx, int ny,
+                        Partial* out) {
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ Partial red[FIN_THREADS / 32];
     __shared__ Partial cta_result;
@@ -730,8 +733,8 @@ __global__ void finalize_cluster_kernel(const Partial* __restrict__ parts, int n
 }
 
 __global__ void __launch_bounds__(FIN_THREADS)
-finalize_small_kernel(const Partial* __restrict__ parts, int nblocks, int nx, int ny,
-                      Partial* __restrict__ out) {
+finalize_small_kernel(const Partial* parts, int nblocks, int nx, int ny,
+                      Partial* out) {
     __shared__ Partial red[FIN_THREADS / 32];
     const long long N = (long long)nx * ny;
     double tm = -1.0; long long ag = N; int mn = ny, mx = -1;
@@ -752,8 +755,8 @@ finalize_small_kernel(const Partial* __restrict__ parts, int nblocks, int nx, in
     }
 }
 
-__global__ void extract_col_kernel(const double* __restrict__ T, int nx, int ny,
-                                   const Partial* __restrict__ glob, double* __restrict__ col) {
+__global__ void extract_col_kernel(const double* T, int nx, int ny,
+                                   const Partial* glob, double* col) {
     const int y = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_trigger();
     pdl_wait();

@@ -229,6 +229,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // of finished blocks before this kernel ends.  pdl_trigger allows that;
 // pdl_wait, before a kernel's first access to global memory, waits until every
 // earlier kernel of the stream has completed and its writes are visible.
+// What such a kernel wrote is read by plain loads, which stay behind the wait:
+// __ldg and const __restrict__ promise memory that nobody writes while this
+// kernel runs, and it runs while its producer still does.
 __device__ __forceinline__ void pdl_trigger() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
