@@ -141,11 +141,11 @@ bool tensor_map_pixel_pairs_bf16(const void* base, int W, int H, int B, int box_
 // ---- launch of one temporally blocked step ---------------------------------
 namespace {
 
-template <int K, bool TMA, bool REDUCE, bool SQ>
+template <int K, bool TMA, bool REDUCE, int SQM>
 cudaError_t launch_t(const double* Tin, double* Tout, const Coef& c, const LaserSub* las,
                      Partial* ring, Workspace* ws, Partial* ref_out, long long ref_nparts,
                      int rows, cudaStream_t stream, const RowWindow* win, int parts_cap) {
-    auto kern = advance_kernel<K, TMA, REDUCE, SQ>;
+    auto kern = advance_kernel<K, TMA, REDUCE, SQM>;
     const size_t smem = TMA ? ADV_SMEM_BYTES : 0;
 
     static int occ[64] = {0};
@@ -244,39 +244,45 @@ cudaError_t launch_t(const double* Tin, double* Tout, const Coef& c, const Laser
     return launch_chained(kern, grid, ADV_WARPS * 32, smem, stream, map, p);
 }
 
-template <int K, bool SQ>
+template <int K, int SQM>
 cudaError_t launch_k2(bool tma, bool reduce, const double* Tin, double* Tout, const Coef& c,
                       const LaserSub* las, Partial* ring, Workspace* ws, Partial* ref_out,
                       long long ref_nparts, int rows, cudaStream_t s, const RowWindow* w,
                       int cap) {
-    if (tma) {
-        const cudaError_t e = reduce
-            ? launch_t<K, true, true, SQ>(Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows,
-                                          s, w, cap)
-            : launch_t<K, true, false, SQ>(Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows,
-                                           s, w, cap);
-        if (e != cudaErrorNotSupported) return e;
-        // tensor map unavailable: fall through to the direct-load kernel
+    if constexpr (SQM != 3) {
+        if (tma) {
+            const cudaError_t e = reduce
+                ? launch_t<K, true, true, SQM>(Tin, Tout, c, las, ring, ws, ref_out, ref_nparts,
+                                               rows, s, w, cap)
+                : launch_t<K, true, false, SQM>(Tin, Tout, c, las, ring, ws, ref_out, ref_nparts,
+                                                rows, s, w, cap);
+            if (e != cudaErrorNotSupported) return e;
+            // tensor map unavailable: fall through to the direct-load kernel
+        }
     }
     return reduce
-        ? launch_t<K, false, true, SQ>(Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows, s, w,
-                                       cap)
-        : launch_t<K, false, false, SQ>(Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows, s,
-                                        w, cap);
+        ? launch_t<K, false, true, SQM>(Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows, s,
+                                        w, cap)
+        : launch_t<K, false, false, SQM>(Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows, s,
+                                         w, cap);
 }
 
 // Square cells (ax == ay, the same comparison the kernels make) take the
-// one-Laplacian form of the cell update.
+// one-Laplacian form of the cell update; Tamb != Tsub on direct loads takes
+// form 3 (WarpStrip).
 template <int K>
 cudaError_t launch_k(bool tma, bool reduce, const double* Tin, double* Tout, const Coef& c,
                      const LaserSub* las, Partial* ring, Workspace* ws, Partial* ref_out,
                      long long ref_nparts, int rows, cudaStream_t s, const RowWindow* w,
                      int cap) {
+    if (!tma && !c.same_T)
+        return launch_k2<K, 3>(tma, reduce, Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows,
+                               s, w, cap);
     return c.ax == c.ay
-        ? launch_k2<K, true>(tma, reduce, Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows,
-                             s, w, cap)
-        : launch_k2<K, false>(tma, reduce, Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows,
-                              s, w, cap);
+        ? launch_k2<K, 1>(tma, reduce, Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows,
+                          s, w, cap)
+        : launch_k2<K, 0>(tma, reduce, Tin, Tout, c, las, ring, ws, ref_out, ref_nparts, rows,
+                          s, w, cap);
 }
 
 }  // namespace

@@ -238,7 +238,11 @@ static_assert(offsetof(RedSmem<3>, box) % 16 == 0 && sizeof(RedSmem<3>) % 16 == 
 // row length and a 16-byte aligned field.
 // SQM: which cell_net form the strip uses — 0 the general one, 1 the
 // square-cell one, 2 the field's own (h.sq), chosen per task (the batched
-// kernel, whose fields differ).
+// kernel, whose fields differ); 3: direct loads of a field with Tamb != Tsub,
+// which runs in the general body only and fetches the row factors only in
+// boxes that meet the source (with the shuffle in every row of every box 12
+// steps of a 6001 x 3500 field took 1035 us, without it 1010; in the other
+// forms the branch costs more than the shuffle: 8192^2 by 3 %).
 template <int K, bool TMA, bool REDUCE, bool BULK = false, int SQM = 0>
 struct WarpStrip {
     static constexpr int V = ADV_V;
@@ -262,6 +266,7 @@ struct WarpStrip {
     bool mlane;                          // this lane is a mirror lane
     int msrc;                            // lane whose cells this lane mirrors (own lane if none)
     bool fast_ok;                        // the task may use the fast body at all
+    bool src_now;                        // the general body's box meets the source (SQM 3)
     bool incl;                           // this task also examines values equal to the lane peak
 
     // Source factors of a task that meets the source: the column factors of
@@ -401,7 +406,13 @@ struct WarpStrip {
             const bool src_box = src_strip && j + 1 >= p.band_lo && j - K <= p.band_hi;
             const bool interior = fast_ok && j - K >= 1 && j + 1 <= ny - 2;
             const bool fast = interior && !src_box;
-            if (fast && j < jend) {
+            if constexpr (SQM == 3) {
+                src_now = src_box;
+                if (src_box) fill_rows(j, true);
+                general_row<0>(j, st, jlast);
+                general_row<1>(j + 1, st, jlast);
+                general_row<2>(j + 2, st, jlast);
+            } else if (fast && j < jend) {
                 if constexpr (SQM == 2) {
                     if (h.sq) fast_box<true, false>(j, st);
                     else      fast_box<false, false>(j, st);
@@ -693,14 +704,15 @@ struct WarpStrip {
                 if (xl + v == nx - 1) R[v] = ce[v];
             }
         }
-        const double rf = __shfl_sync(0xffffffffu, srcf[K * V], 3 * (T - 1) + P);
+        double rf = 0.0;
+        if (SQM != 3 || src_now) rf = __shfl_sync(0xffffffffu, srcf[K * V], 3 * (T - 1) + P);
         const bool src = rf != 0.0;
         double S[V] = {0.0, 0.0, 0.0, 0.0};
         if (src) {
 #pragma unroll
             for (int v = 0; v < V; ++v) S[v] = src_product(rf, srcf[(T - 1) * V + v]);
         }
-        if (c.same_T) {
+        if (SQM != 3 && c.same_T) {
 #pragma unroll
             for (int v = 0; v < V; ++v)
                 nv[v] = src ? gcore_src(ce[v], L[v], R[v], up[v], dn[v], S[v])
@@ -920,7 +932,7 @@ struct WarpStrip {
 template <int K>
 struct AdvOcc { static constexpr int min_ctas = 3; };
 
-template <int K, bool TMA, bool REDUCE, bool SQ>
+template <int K, bool TMA, bool REDUCE, int SQM>
 __global__ void __launch_bounds__(ADV_WARPS * 32, AdvOcc<K>::min_ctas)
 advance_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ AdvParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -942,8 +954,8 @@ advance_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ 
         __syncwarp();
     }
 
-    WarpStrip<K, TMA, REDUCE, false, SQ ? 1 : 0> ws(p, &map, stages, bars, lane,
-                                                    &s_red[REDUCE ? wid : 0]);
+    WarpStrip<K, TMA, REDUCE, false, SQM> ws(p, &map, stages, bars, lane,
+                                             &s_red[REDUCE ? wid : 0]);
     pdl_trigger();
     pdl_wait();
     if (p.tasks) {
