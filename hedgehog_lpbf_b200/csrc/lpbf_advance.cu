@@ -327,9 +327,16 @@ int resolve_depth(const lpbf_b200_opts* o) {
 // cells), unless the caller asks for a depth or task height of the launch
 // path: measured per step against the launch path, 1.0 : 20 us at 240 x 120,
 // 1.5 : 16 at 512^2, 2.9 : 16 at 1021 x 763, 4.7 : 20 at 1344 x 1216; a call
-// of 16 steps takes 38 us at 512^2, a call of one step one launch either way.
+// of 16 steps takes 38 us at 512^2.  From 2^20 cells, calls too short to pay
+// for filling its tiles stay on the launch path, in one launch either way: one
+// step (us, resident : launch path: 1000^2 13.9 : 15.4, 1024^2 22.8 : 15.5,
+// 1440^2 25.1 : 16.8), and two where the tiles fit with a halo of one only, so
+// that they would trade rims between the two (2000 x 1000 43.5 : 29.9; with a
+// halo of two 1344 x 1216 28.6 : 29.3; 1000^2 with one 25.0 : 27.6).
 bool resident(const lpbf_b200_opts* o, int nx, int ny, int n_steps, ResPlan* pl) {
-    return o->phys == 0 && o->depth <= 0 && o->rows <= 0 && resident_plan(nx, ny, n_steps, pl);
+    if (o->phys != 0 || o->depth > 0 || o->rows > 0 || !resident_plan(nx, ny, n_steps, pl))
+        return false;
+    return n_steps > 2 || (long long)nx * ny < (1ll << 20) || (n_steps == 2 && pl->K > 1);
 }
 
 bool valid_const(const StepConst* k) {
