@@ -41,7 +41,8 @@ struct Workspace {
     unsigned int err;              // error word
     unsigned int tasks;            // dynamic task counter
     unsigned int barrier;          // arrivals of the resident kernel's final fold
-    unsigned int pad[60];
+    unsigned int wait_ns;          // limit of the resident kernel's waits; 0: RES_WAIT_NS
+    unsigned int pad[59];
     Partial parts[WS_PARTS];
     unsigned int flags[160 * 8];   // zero between launches
 };

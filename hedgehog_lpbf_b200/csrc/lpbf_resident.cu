@@ -133,6 +133,7 @@ cudaError_t launch_resident(const ResPlan& pl, const double* Tin, double* Tout, 
     p.counter = &ws->counter;
     p.barrier = &ws->barrier;
     p.err = &ws->err;
+    p.wait_ns = &ws->wait_ns;
     p.n_steps = n_steps;
     p.K = pl.K;
     p.nblocks = (n_steps + pl.K - 1) / pl.K | 1;      // odd: the result is in Tout

@@ -76,6 +76,7 @@ struct ResParams {
     unsigned int* counter;         // exit ticket, zero between launches
     unsigned int* barrier;         // arrivals of the final fold, zero between launches
     unsigned int* err;
+    const unsigned int* wait_ns;   // Workspace::wait_ns
     int n_steps, nblocks, K;       // K: most steps of a block
     int gx, gy;                    // tiles per row and column of tiles
     int hx, hy;                    // halo columns and rows held per side
@@ -115,12 +116,15 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
 __device__ __forceinline__ void st_release(unsigned int* p, unsigned int v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
-// Wait until *p >= want, at most RES_WAIT_NS.
-__device__ __forceinline__ bool res_wait(const unsigned int* p, unsigned int want) {
+// Wait until *p >= want, at most *limit ns (0: RES_WAIT_NS).
+__device__ __forceinline__ bool res_wait(const unsigned int* p, unsigned int want,
+                                         const unsigned int* limit) {
     if (ld_acquire(p) >= want) return true;
     const uint64_t t0 = globaltimer_ns();
+    const unsigned int w = *limit;
+    const uint64_t ns = w ? w : RES_WAIT_NS;
     while (ld_acquire(p) < want)
-        if (globaltimer_ns() - t0 > RES_WAIT_NS) return false;
+        if (globaltimer_ns() - t0 > ns) return false;
     return true;
 }
 
@@ -489,7 +493,7 @@ resident_kernel(const __grid_constant__ ResParams p) {
         if (tid < 9 && tid != 4) {
             const int ox = bx + tid % 3 - 1, oy = by + tid / 3 - 1;
             if (ox >= 0 && ox < p.gx && oy >= 0 && oy < p.gy &&
-                !res_wait(p.flags + (oy * p.gx + ox) * RES_FLAG_STRIDE, (unsigned)b))
+                !res_wait(p.flags + (oy * p.gx + ox) * RES_FLAG_STRIDE, (unsigned)b, p.wait_ns))
                 s_flag = 0;
         }
         src = __syncthreads_or(any_row);
@@ -528,7 +532,7 @@ resident_kernel(const __grid_constant__ ResParams p) {
         if (tid == 0) {
             __threadfence();
             atomicAdd(p.barrier, 1u);
-            s_flag = failed ? 0 : (res_wait(p.barrier, gridDim.x) ? 1 : 0);
+            s_flag = failed ? 0 : (res_wait(p.barrier, gridDim.x, p.wait_ns) ? 1 : 0);
             if (!s_flag) atomicOr(p.err, 1u);
         }
         __syncthreads();
