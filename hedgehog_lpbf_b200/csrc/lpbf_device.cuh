@@ -300,5 +300,11 @@ __device__ __forceinline__ p2 p2_sub(p2 a, p2 b) {
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+// Rounded towards +infinity.
+__device__ __forceinline__ p2 p2_sub_up(p2 a, p2 b) {
+    p2 r;
+    asm("sub.rp.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 
 }  // namespace lpbf_b200

@@ -526,14 +526,16 @@ struct FkStrip {
             }
             if constexpr (REDUCE) {
                 // the largest of the four cells against the box threshold (NaN
-                // never wins a maximum); pairs by the sign of their exact
-                // difference
+                // never wins a maximum); pairs by the sign of their difference.
+                // Its lo part is rounded up: where it all but cancels a step of
+                // hi, a cell above the threshold must not come out equal to it
+                // (one just below may pass: the exact pass decides)
                 const float th = own ? thr_h[T - 1] : INFINITY;
                 bool rh;
                 if constexpr (COMP) {
                     const p2 tp = p2_pack(th, th), tq = p2_pack(thr_l[T - 1], thr_l[T - 1]);
-                    const p2 e0 = p2_add(p2_sub(oh[0], tp), p2_sub(ol[0], tq));
-                    const p2 e1 = p2_add(p2_sub(oh[1], tp), p2_sub(ol[1], tq));
+                    const p2 e0 = p2_add(p2_sub(oh[0], tp), p2_sub_up(ol[0], tq));
+                    const p2 e1 = p2_add(p2_sub(oh[1], tp), p2_sub_up(ol[1], tq));
                     rh = fmaxf(fmaxf(p2_a(e0), p2_b(e0)), fmaxf(p2_a(e1), p2_b(e1))) > 0.0f;
                 } else {
                     rh = fmaxf(fmaxf(p2_a(oh[0]), p2_b(oh[0])),
