@@ -272,6 +272,12 @@ struct ExtStrip {
     int py, px, mn, mx;
 };
 
+// What a cell must exceed to change the lane's peak or a molten row.  A melt
+// threshold that is NaN (no cell is molten) leaves the peak's.
+__device__ __forceinline__ double ext_threshold(const ExtStrip& s, double Tm) {
+    return s.own ? (Tm < s.tm ? Tm : s.tm) : INFINITY;
+}
+
 // Row y (clamped to the field) of the lane's two columns.  VEC (rows on
 // 16-byte boundaries, nx even): a pair lies wholly on or off the field; one
 // off it takes the edge cell twice.
@@ -385,7 +391,7 @@ __device__ __forceinline__ void ext_block(const double* Tin,
                 s.mn = min(s.mn, y + __ffs(rows) - 1);
                 s.mx = max(s.mx, y + 31 - __clz(rows));
             }
-            s.thr = s.own ? (s.tm < p.Tm ? s.tm : p.Tm) : INFINITY;
+            s.thr = ext_threshold(s, p.Tm);
         }
     }
 }
@@ -439,7 +445,7 @@ ext_step_kernel(const double* Tin, double* Tout,
         s.own_b = s.own && s.xb < nx;
         const int y0 = chunk * p.H;
         s.y1 = min(y0 + p.H, ny);
-        s.thr = s.own ? (s.tm < p.Tm ? s.tm : p.Tm) : INFINITY;
+        s.thr = ext_threshold(s, p.Tm);
         const bool src_strip = k.q_scale != 0.0 && xs + 32 * EXT_V > p.bandx_lo &&
                                xs <= p.bandx_hi;
         double Q[EXT_R][2];
