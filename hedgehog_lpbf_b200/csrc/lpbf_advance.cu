@@ -323,16 +323,18 @@ int resolve_depth(const lpbf_b200_opts* o) {
     return o->depth > 0 ? std::min(o->depth, 4) : AUTO_DEPTH;
 }
 
-// The resident kernel runs every field whose tiles fit (up to about 1.9 M
-// cells), unless the caller asks for a depth or task height of the launch
-// path: measured per step against the launch path, 1.0 : 20 us at 240 x 120,
-// 1.5 : 16 at 512^2, 2.9 : 16 at 1021 x 763, 4.7 : 20 at 1344 x 1216; a call
-// of 16 steps takes 38 us at 512^2.  From 2^20 cells, calls too short to pay
-// for filling its tiles stay on the launch path, in one launch either way: one
-// step (us, resident : launch path: 1000^2 13.9 : 15.4, 1024^2 22.8 : 15.5,
-// 1440^2 25.1 : 16.8), and two where the tiles fit with a halo of one only, so
-// that they would trade rims between the two (2000 x 1000 43.5 : 29.9; with a
-// halo of two 1344 x 1216 28.6 : 29.3; 1000^2 with one 25.0 : 27.6).
+// The resident kernel runs every field whose tiles fit (up to about 2 M cells
+// on 148 SMs, by shape), unless the caller asks for a depth or task height of
+// the launch path: us per step in calls of 128, against the launch path,
+// 1.07 : 14.2 at 240 x 120, 1.6 : 12.5 at 512^2, 3.1 : 19 at 1021 x 763,
+// 4.9 : 13.4 at 1344 x 1216, 5.9 : 13.7 at 1440^2; a call of 16 steps takes
+// 35 us at 512^2 and 113 at 1440^2 (launch path 201 and 225).  From 2^20
+// cells, calls too short to pay for filling its tiles stay on the launch path,
+// in one launch either way: one step (us, resident : launch path: 1000^2
+// 13.9 : 15.4, 1024^2 22.8 : 15.5, 1440^2 25.1 : 16.8), and two where the
+// tiles fit with a halo of one only, so that they would trade rims between the
+// two (2000 x 1000 43.5 : 29.9; with a halo of two 1344 x 1216 28.6 : 29.3;
+// 1000^2 with one 25.0 : 27.6).
 bool resident(const lpbf_b200_opts* o, int nx, int ny, int n_steps, ResPlan* pl) {
     if (o->phys != 0 || o->depth > 0 || o->rows > 0 || !resident_plan(nx, ny, n_steps, pl))
         return false;

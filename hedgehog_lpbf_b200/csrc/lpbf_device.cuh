@@ -110,15 +110,6 @@ __device__ __forceinline__ double cell_update(double T, double L, double R,
     return __dadd_rn(T, __dsub_rn(__dadd_rn(inc, S_dt), loss_dt(T, c)));
 }
 
-// Gaussian source increment at column x of a row whose (y - y_l)^2 is dy2.
-__device__ __forceinline__ double source_dt(int x, double dy2, const LaserSub& l,
-                                            const Coef& c) {
-    const double dxl = __dsub_rn(__dmul_rn((double)x, c.dx), l.x_l);
-    const double r2 = __dadd_rn(__dmul_rn(dxl, dxl), dy2);
-    if (r2 >= c.r2_cut) return 0.0;
-    return l.cs * exp(__dmul_rn(c.m2r, r2));
-}
-
 // ---- Partial combine: larger T wins, equal T -> smaller index ------------
 __device__ __forceinline__ void partial_take(double& tm, long long& ag, int& mn, int& mx,
                                              double t2, long long a2, int mn2, int mx2) {

@@ -146,8 +146,8 @@ __device__ __forceinline__ void fk_cell(float th, float tl, float Lh, float Ll, 
 // increment's fused chain (SQ: one Laplacian (R + L) + (U + D) - 4T).  The
 // Laplacian of a uniform field is exactly zero and its loss at Tamb far below
 // half an ulp of T, so a uniform field at Tamb stays exactly uniform.
-// SRC: the cell's source increment S is added to the net change before T.
-template <bool SQ, bool SRC>
+// The cell's source increment S is added to the net change before T.
+template <bool SQ>
 __device__ __forceinline__ float f32_cell(float t, float L, float R, float U, float D, float S,
                                           const FkCoef& f) {
     const float t2 = __fmul_rn(t, t);
@@ -162,8 +162,7 @@ __device__ __forceinline__ float f32_cell(float t, float L, float R, float U, fl
         const float ly = fmaf(-2.0f, t, __fadd_rn(U, D));
         net = fmaf(f.ax, lx, fmaf(f.ay, ly, -loss));
     }
-    if constexpr (SRC) net = __fadd_rn(net, S);
-    return __fadd_rn(t, net);
+    return __fadd_rn(t, __fadd_rn(net, S));
 }
 
 // (a.hi, a.lo) > (b.hi, b.lo) for canonical pairs.
@@ -382,7 +381,7 @@ struct FkStrip {
             }
 #pragma unroll
             for (int v = 0; v < V; ++v)
-                oh[v] = f32_cell<SQ, true>(ch[v], L[v], R[v], uh[v], dh[v], S[v], p.f);
+                oh[v] = f32_cell<SQ>(ch[v], L[v], R[v], uh[v], dh[v], S[v], p.f);
         } else {
             const float Lh0 = __shfl_up_sync(0xffffffffu, ch[V - 1], 1);
             const float Ll0 = __shfl_up_sync(0xffffffffu, cl[V - 1], 1);

@@ -93,8 +93,8 @@ inline cudaError_t launch_chained(Args&&... args) {
 }
 
 // Rows whose source term can be non-zero in any of the K substeps (a
-// superset: the kernel decides exactly, this only routes rows to the general
-// body).  Empty when every substep has the beam off.
+// superset: the kernel decides exactly, this only routes boxes to the bodies
+// with the source).  Empty when every substep has the beam off.
 inline void laser_band(const Coef& c, const LaserSub* las, int K, int* lo, int* hi, int* xlo,
                 int* xhi) {
     int blo = 1 << 30, bhi = -(1 << 30), cxlo = 1 << 30, cxhi = -(1 << 30);
@@ -136,7 +136,7 @@ cudaError_t launch_advance(int K, const double* Tin, double* Tout, const Coef& c
                            cudaStream_t stream, const RowWindow* win = nullptr,
                            int parts_cap = MAX_CTAS * KMAX);
 
-// Many steps of a field small enough to stay in shared memory in one launch
+// Many steps of a field small enough to stay in registers in one launch
 // (lpbf_resident.cuh).  resident_plan: false when the field does not fit;
 // `steps` is the most steps of one launch.  launch_resident advances n_steps
 // (<= steps) from Tin into Tout; Tin_rw is Tin, which carries the tiles' rims
@@ -148,8 +148,8 @@ cudaError_t launch_resident(const ResPlan& pl, const double* Tin, double* Tout, 
                             const Coef& c, const LaserSub* las, int n_steps, Partial* ring,
                             Workspace* ws, cudaStream_t stream);
 
-// Extended-physics (phys == 1) single step, one thread per cell, with the
-// same reduction outputs as launch_advance.
+// Extended-physics (phys == 1) single step (a warp per strip of rows, four
+// rows per block), with the same reduction outputs as launch_advance.
 cudaError_t launch_ext_step(const double* Tin, double* Tout, const StepConst& k,
                             int bc, double T_edge, double Tm, Partial* ring,
                             Workspace* ws, Partial* ref_out, long long ref_nparts,

@@ -302,9 +302,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
 
-// Epilogue of 16 accumulator columns (channels c0 .. c0 + 15) of pixel p.
-// GELU: bias, pre-activation and activation out (bf16); LINEAR: channel 0
-// plus bias (fp32); DGELU: times gelu'(pre_in) (bf16).
 // DGELU: the pre-activations of epilogue16's 16 channels (loaded ahead of the
 // accumulator's wait where there is one).
 template <int N, int EPI>
@@ -322,6 +319,9 @@ __device__ __forceinline__ void load_pre16(const ConvArgs& a, size_t p, int c0, 
     }
 }
 
+// Epilogue of 16 accumulator columns (channels c0 .. c0 + 15) of pixel p.
+// GELU: bias, pre-activation and activation out (bf16); LINEAR: channel 0
+// plus bias (fp32); DGELU: times gelu'(pre_in), given in w (bf16).
 template <int N, int EPI>
 __device__ __forceinline__ void epilogue16(const ConvArgs& a, size_t p, int c0, const float* v,
                                            const float* bias, const uint32_t (&w)[8]) {

@@ -11,11 +11,14 @@
 // laser at the middle of those steps in units of 100 um (x and y, clamped to
 // +-8).  Output: (T after 16 steps - T) / 100 K.
 //
-// Weight gradients are a tensor-core GEMM over pixels: rows are (tap, input
-// channel) pairs plus one all-ones row (the bias), columns the output
-// channels, and K runs over 64-pixel blocks staged transposed in shared
-// memory (double-buffered, one mbarrier per stage); per-CTA partials are
-// summed by a second kernel in a fixed order (deterministic).
+// Weight gradients: the 32 -> 32 layers stream rows through tcgen05, the 4 -> 32
+// and 32 -> 1 layers through warp-level MMAs (lpbf_surrogate.cu).  Here is the
+// general form, which any other form or an unaligned buffer takes: a
+// tensor-core GEMM over pixels, rows (tap, input channel) pairs plus one
+// all-ones row (the bias), columns the output channels, K over 64-pixel blocks
+// staged transposed in shared memory (double-buffered, one mbarrier per
+// stage).  In all of them per-CTA partials are summed by a second kernel in a
+// fixed order (deterministic).
 //
 // Network blob (device, caller-allocated, lpbf_b200_sg_net_bytes): fp32
 // master parameters, gradients, AdamW moments m and v (each

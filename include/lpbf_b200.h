@@ -12,9 +12,10 @@
  *   lpbf_b200_advance   the per-step loop of GpuStepTask::execute
  *                       (include/gpu_step_task.hpp:149-197): step + reduce +
  *                       finalize for `n_steps` Ticks of a plan, in
- *                       ceil(n_steps / depth) launches (fields of up to
- *                       about 1.9 M cells at automatic depth: one per 256
- *                       steps) instead of 2-4 launches per step.
+ *                       ceil(n_steps / depth) launches (small and middling
+ *                       fields at automatic depth: one per up to 256 steps,
+ *                       see lpbf_b200_advance_launches) instead of 2-4
+ *                       launches per step.
  * ---------------------------------------------------------------------------
  */
 #ifndef LPBF_B200_H
@@ -90,7 +91,9 @@ int lpbf_b200_advance(double* T_a, double* T_b, const StepConst* k,
                       cudaStream_t stream, int* result_in_b);
 
 /* Number of launches lpbf_b200_advance issues for these arguments (with a
- * workspace; it depends on the current device). */
+ * workspace).  At automatic depth a field whose tiles fit the device's SMs
+ * advances up to 256 steps per launch: on 148 SMs up to about 2 M cells, by
+ * its shape (1440 x 1440 fits, 1500 x 1400 and 130 x 15000 do not). */
 int lpbf_b200_advance_launches(int nx, int ny, int n_steps, const lpbf_b200_opts* opts);
 
 /* A row strip of a larger field: the buffers hold rows row0 .. row0+k->ny-1
