@@ -958,6 +958,10 @@ wgrad_row_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
                         gs + px * 64 + ((((lane >> 3) ^ (px >> 1)) & 3) << 4) + (lane & 7) * 2);
                     bsum += __uint_as_float(uint32_t(v) << 16);
                 }
+                // the reads before the copy that refills the slot: the arrival
+                // alone does not order them against the copy engine (bias
+                // gradients then differed from run to run)
+                fence_smem_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&gempty[gg % WR_GS]);
             }
