@@ -86,8 +86,8 @@ def measured_peaks():
 # and the FP64 pipe's share of active cycles (4096^2 --set full capture of
 # the same kernel).
 ADVANCE_PROFILE = {
-    3: {"dram_bytes": 1.13944e9, "dram_read_bytes": 0.60274e9, "dram_write_bytes": 0.53670e9,
-        "fp64_pipe": 0.539, "issue_active": 0.495, "limiter": "fp64_pipe_latency",
+    3: {"dram_bytes": 1.14119e9, "dram_read_bytes": 0.60357e9, "dram_write_bytes": 0.53762e9,
+        "fp64_pipe": 0.547, "issue_active": 0.502, "limiter": "fp64_pipe_latency",
         "source": "profiles/advance_kernel_8192.md"},
 }
 
